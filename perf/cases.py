@@ -451,6 +451,12 @@ def _sky(s, c, ph):
 
 
 def _rk4(rhs, y, k1, h):
+    """One step from y with k1 = rhs(y): the new state and the last stage's derivative (lists of duals, or one tensor)."""
+    if isinstance(y, torch.Tensor):
+        k2 = rhs(y + k1 * (0.5 * h))
+        k3 = rhs(y + k2 * (0.5 * h))
+        k4 = rhs(y + k3 * h)
+        return y + (k1 + 2 * (k2 + k3) + k4) * (h / 6), k4
     k2 = rhs([p + k * (0.5 * h) for p, k in zip(y, k1)])
     k3 = rhs([p + k * (0.5 * h) for p, k in zip(y, k2)])
     k4 = rhs([p + k * h for p, k in zip(y, k3)])
@@ -489,11 +495,11 @@ def _exact_frame(case, v):
         E, L, pr, pth = _kerr_start(a, s0 + z, c0 + z, d, nr, nt, nph)
         Q = pth * pth + c0 * c0 * (L * L / (s0 * s0) - a * a * E * E)
     if adaptive:
-        y = [d + z, s0 + z, c0 + z, az + z, pr, pth]
+        y = torch.stack([d + z, s0 + z, c0 + z, az + z, pr, pth])
 
         def rhs(y):
             k = _kerr_rhs(y[0], y[1], y[2], y[4], y[5], E, L, a)
-            return [k[0], y[2] * k[1], -y[1] * k[1], k[2], k[3], k[4]]
+            return torch.stack([k[0], y[2] * k[1], -y[1] * k[1], k[2], k[3], k[4]])
 
         lo, hi = (2 * (1 + math.cos(2 / 3 * math.acos(q * a))) for q in (-1, 1))
         xi = L / E
@@ -507,22 +513,22 @@ def _exact_frame(case, v):
         r_cap = torch.where((ok | (a <= 1e-7)) & (Q >= 0), torch.clamp(r_c - 0.05, max=r_in), z)
         k1, h = rhs(y), 0.1 * y[0]
     elif kerr:
-        y = [d + z, th0 + z, az + z, pr, pth]
+        y = torch.stack([d + z, th0 + z, az + z, pr, pth])
 
         def rhs(y):
-            return list(_kerr_rhs(y[0], torch.sin(y[1]), torch.cos(y[1]), y[3], y[4], E, L, a))
+            return torch.stack(_kerr_rhs(y[0], torch.sin(y[1]), torch.cos(y[1]), y[3], y[4], E, L, a))
     else:
         ut, up = nt / d, nph / (d * s0)
         f = 1 - 2 / d
-        y = [d + z, th0 + z, az + z, torch.sqrt((nr * nr / f + nt * nt + nph * nph) / f), nr, ut, up]
+        y = torch.stack([d + z, th0 + z, az + z, torch.sqrt((nr * nr / f + nt * nt + nph * nph) / f), nr, ut, up])
 
         def rhs(y):
             r, th, _, ut, ur, uth, uph = y
             f, s, c = 1 - 2 / r, torch.sin(th), torch.cos(th)
-            return [ur, uth, uph, -2 / (r * r * f) * ut * ur,
-                    -f / (r * r) * ut * ut + ur * ur / (r * r * f) + r * f * (uth * uth + s * s * uph * uph),
-                    -2 * ur * uth / r + s * c * uph * uph, -2 * ur * uph / r - 2 * c / s * uth * uph]
-    prev = [] if adaptive else y
+            p, q, g = r * r * f, uph * uph, -2 * ur / r
+            return torch.stack([ur, uth, uph, -2 * ut * ur / p, (ur * ur - (f * ut) ** 2) / p + r * f * (uth * uth + s * s * q),
+                                g * uth + s * c * q, (g - 2 * c / s * uth) * uph])
+    prev = y
     for _ in range(case["max_steps"]):
         r = y[0]
         if adaptive:
@@ -530,9 +536,6 @@ def _exact_frame(case, v):
         else:
             fall = ~torch.isfinite(r) | (r < hcut)
         out = ~fall & (r > 200)
-        if out.any():
-            s, c, ph = (y[1], y[2], y[3]) if adaptive else (torch.sin(y[1]), torch.cos(y[1]), y[2])
-            put(out, _sky(s[out], c[out], ph[out]))
         over = fall | out
         if not adaptive:
             p, q = prev[1] - PI / 2, y[1] - PI / 2
@@ -543,12 +546,14 @@ def _exact_frame(case, v):
                 emit(hit, rc[hit], y[2][hit], L[hit] if kerr else (prev[6] + x * (y[6] - prev[6]))[hit])
             over = over | hit
         if over.any():
+            s, c, ph = (t[out] for t in ((y[1], y[2], y[3]) if adaptive else (torch.sin(y[1]), torch.cos(y[1]), y[2])))
+            put(out, _sky(s, c, ph))
             keep = ~over
-            ids, y, prev = ids[keep], [t[keep] for t in y], [t[keep] for t in prev]
+            ids, y, prev = ids[keep], y[:, keep], prev if adaptive else prev[:, keep]
             if kerr:
                 E, L = E[keep], L[keep]
             if adaptive:
-                Q, r_cap, h, k1 = Q[keep], r_cap[keep], h[keep], [t[keep] for t in k1]
+                Q, r_cap, h, k1 = Q[keep], r_cap[keep], h[keep], k1[:, keep]
             if not ids.numel():
                 break
         if not adaptive:
@@ -560,8 +565,7 @@ def _exact_frame(case, v):
         h = torch.minimum(h, 0.1 * y[0])
         new, k4 = _rk4(rhs, y, k1, h)
         k5 = rhs(new)
-        err = torch.stack([torch.abs(h / 6 * (a4 - a5)) / (1e-6 * (1 + torch.maximum(p.abs(), q.abs())))
-                           for a4, a5, p, q in zip(k4, k5, y, new)]).amax(0)
+        err = (torch.abs(h / 6 * (k4 - k5)) / (1e-6 * (1 + torch.maximum(y.abs(), new.abs())))).amax(0)
         err = torch.where(err <= 1e30, err, torch.full_like(err, 1e30))
         accept = err <= 1
         hit = accept & (y[2] * new[2] < 0) & (new[1] > 0)
@@ -579,14 +583,13 @@ def _exact_frame(case, v):
             emit(over, rc[on], pc[on], L[over])
         h = h * torch.where(err <= 1e-30, torch.full_like(err, 4.0), torch.clamp(0.85 / err ** 0.25, 0.2, 4.0))
         n2 = 1.5 - 0.5 * (new[1] ** 2 + new[2] ** 2)
-        new[1], new[2] = new[1] * n2, new[2] * n2
+        new[1:3] *= n2
         theta = Q - new[2] ** 2 * (L * L / torch.clamp(new[1] ** 2, min=1e-10) - a * a * E * E)
         new[5] = torch.copysign(torch.sqrt(torch.clamp(theta, min=0)), new[5])
-        y = [torch.where(accept, q, p) for p, q in zip(y, new)]
-        k1 = [torch.where(accept, q, p) for p, q in zip(k1, k5)]
+        y, k1 = torch.where(accept, new, y), torch.where(accept, k5, k1)
         if over.any():
             keep = ~over
-            ids, y, k1 = ids[keep], [t[keep] for t in y], [t[keep] for t in k1]
+            ids, y, k1 = ids[keep], y[:, keep], k1[:, keep]
             E, L, Q, r_cap, h = E[keep], L[keep], Q[keep], r_cap[keep], h[keep]
             if not ids.numel():
                 break
