@@ -29,8 +29,9 @@ namespace sgxa {
 SGX_HD float hsqrt(float x) { return sqrtf(x); }
 SGX_HD double hsqrt(double x) { return sqrt(x); }
 // 1/x: PTX rcp.approx.ftz.f32 on the device in FP32 (one SFU instruction, at
-// most 1 ulp from 1/x; the forward kernel's rhs_g does the same), exact
-// elsewhere.
+// most 1 ulp from 1/x; the forward kernel's rhs_g does the same), rcp_newton
+// on the device in FP64 (three FP64 instructions, at most 1 ulp), exact on
+// the host.
 SGX_HD float hrcp(float x) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -40,7 +41,31 @@ SGX_HD float hrcp(float x) {
     return 1.0f / x;
 #endif
 }
-SGX_HD double hrcp(double x) { return 1.0 / x; }
+SGX_HD double hrcp(double x) {
+#if defined(__CUDA_ARCH__)
+    return sgxd::rcp_newton(x);
+#else
+    return 1.0 / x;
+#endif
+}
+SGX_HD float hfma(float a, float b, float c) { return fmaf(a, b, c); }
+SGX_HD double hfma(double a, double b, double c) { return fma(a, b, c); }
+// the sin^2 guard of the right-hand side, max(x, 1e-10); in FP64 on the device
+// an integer comparison (x >= 0)
+template <class T> SGX_HD T hguard(T x) {
+#if defined(__CUDA_ARCH__)
+    if constexpr (std::is_same_v<T, double>) return sgxd::pos_max(x, 1e-10);
+#endif
+    return x < T(1e-10) ? T(1e-10) : x;
+}
+// x / 6, correctly rounded
+template <class T> SGX_HD T hsixth(T x) {
+#if defined(__CUDA_ARCH__)
+    return sgxd::sixth(x);
+#else
+    return x / T(6);
+#endif
+}
 // State layout: y[0..7] = r, theta, phi, p_r, p_theta, psi (swept angle),
 // s = sin(theta), c = cos(theta); derivative layout d[0..6] = dr, dtheta,
 // dphi, dp_r, dp_theta, ds, dc.  theta is integrated for the swept angle and
@@ -157,7 +182,8 @@ template <class T> SGX_HD void ksum7(const T* k1, const T* k2, const T* k3, cons
         return;
     }
 #endif
-    for (int i = 0; i < 7; ++i) ks[i] = (k1[i] + k2[i] * T(2)) + (k3[i] * T(2) + k4[i]);
+    // fused: a doubling written as a sum is one more instruction in FP64
+    for (int i = 0; i < 7; ++i) ks[i] = hfma(T(2), k2[i], k1[i]) + hfma(T(2), k3[i], k4[i]);
 }
 
 // The right-hand side in Carter's separated form (the same Hamiltonian as
@@ -167,24 +193,40 @@ template <class T> SGX_HD void ksum7(const T* k1, const T* k2, const T* k3, cons
 //   dp_r  = (r N / Sigma + (M - r)(p_r^2 + Q^2) + 2 E r Q) / Sigma,
 //   dp_th = -sin(th) cos(th) (a^2 N / Sigma - U (2 a E + U)) / Sigma.
 // plus ds = cos(th) dth, dc = -sin(th) dth, with sin(th), cos(th) read from
-// the state.  Operation for operation the forward kernel's rhs_g7
-// (sgx_diff_impl.cuh).
+// the state.  In FP32 operation for operation the forward kernel's rhs_g7
+// (sgx_diff_impl.cuh), in FP64 that is this function.
 template <class T>
 SGX_HD void rhs7(const T* y, T E, T L, T a, T M, T* d) {
     const T st = y[6], ct = y[7];
     const T r = y[0];
     const T a2 = a * a;
     const T s2 = st * st;
-    const T ss = s2 < T(1e-10) ? T(1e-10) : s2;
+    const T ss = hguard(s2);
     const T r2 = r * r;
     const T r2a2 = r2 + a2;
-    const T Sig = r2 + a2 * (ct * ct);
+    T Sig;
+    if constexpr (std::is_same_v<T, double>) Sig = r2a2 + a2 * (ct * ct - T(1));
+    else Sig = r2 + a2 * (ct * ct);
     const T Del = r2a2 - (T(2) * M) * r;
     const T aE = a * E;
     const T P = r2a2 * E - a * L;
     const T W = L - aE * s2;
     const T iS = hrcp(Sig), iD = hrcp(Del), is2 = hrcp(ss);
     const T Q = P * iD, U = W * is2;
+    if constexpr (std::is_same_v<T, double>) {
+        // the same terms in fewer instructions (FP64 is bound by their number;
+        // as the tracer's FP64 right-hand side)
+        const T Dpr = Del * y[3];
+        const T NiS = (((Dpr * y[3] + y[4] * y[4]) - P * Q) + W * U) * iS;
+        d[0] = Dpr * iS;
+        d[1] = y[4] * iS;
+        d[2] = (a * Q + U) * iS;
+        d[3] = (r * ((T(2) * E) * Q + NiS) + (M - r) * (Q * Q + y[3] * y[3])) * iS;
+        d[4] = (iS * (st * ct)) * (U * (T(2) * aE + U) - a2 * NiS);
+        d[5] = ct * d[1];
+        d[6] = -(st * d[1]);
+        return;
+    }
     d[0] = Del * y[3] * iS;
     d[1] = y[4] * iS;
     d[2] = (a * Q + U) * iS;
@@ -352,7 +394,7 @@ template <class T> SGX_HD void step(const T* y, T E, T L, T a, T M, T h, bool fa
     rhs7(t, E, L, a, M, k3);
     for (int i = 0; i < 7; ++i) t[sidx(i)] = y[sidx(i)] + k3[i] * he;
     rhs7(t, E, L, a, M, k4);
-    const T h6 = he / T(6);
+    const T h6 = hsixth(he);
     for (int i = 0; i < 7; ++i) o[sidx(i)] = y[sidx(i)] + ((k1[i] + k2[i] * T(2)) + (k3[i] * T(2) + k4[i])) * h6;
     const T n = T(1.5) - T(0.5) * (o[6] * o[6] + o[7] * o[7]);
     o[6] = o[6] * n;
@@ -381,7 +423,7 @@ template <class T> SGX_HD void step_vjp(const T* y, T E, T L, T a, T M, T h, boo
     rhs7(y3, E, L, a, M, k3);
     stage7(y, k3, he, y4);
     rhs7(y4, E, L, a, M, k4);
-    const T h6 = he / T(6);
+    const T h6 = hsixth(he);
     T ks[7];
     ksum7(k1, k2, k3, k4, ks);
     // RK4 output before and after the renormalisation of (s, c)

@@ -69,11 +69,11 @@ template <class T> struct DiffBufs {
 
 template <class S> __device__ __forceinline__ S selv(bool c, const S& a, const S& b) { return c ? a : b; }
 
-// 1/x of the right-hand side: the SFU reciprocal in FP32 (sgxa::hrcp alike),
-// a division in FP64 and for dual numbers.
+// 1/x of the right-hand side: the SFU reciprocal in FP32, rcp_newton in FP64
+// (sgxa::hrcp alike), a division for dual numbers.
 template <class S> __device__ __forceinline__ S rcp_g(const S& x) {
     if constexpr (std::is_same_v<S, float>) return DM<float>::rcp_fast(x);
-    else if constexpr (std::is_same_v<S, double>) return 1.0 / x;
+    else if constexpr (std::is_same_v<S, double>) return rcp_newton(x);
     else {
         using T = decltype(value_of(x));
         return S(T(1)) / x;
@@ -94,6 +94,7 @@ template <class S> __device__ __forceinline__ S smooth01(const S& x) {
 // equations.
 template <class S, class T>
 __device__ __forceinline__ void rhs_g7(const S* y, const S& E, const S& L, const S& a, T M, S* d) {
+    if constexpr (std::is_same_v<S, double>) return sgxa::rhs7<double>(y, E, L, a, M, d);
     const S& st = y[6];
     const S& ct = y[7];
     const S r = y[0];
@@ -152,7 +153,7 @@ __device__ __forceinline__ void step_g(const S* y, const S& E, const S& L, const
         rhs_g7(t, E, L, a, M, k3);
         axpy(k3, he);
         rhs_g7(t, E, L, a, M, k4);
-        const float h6 = he / 6.0f;
+        const float h6 = sixth(he);
         const F2 two = f2(2.0f, 2.0f), hp = f2(h6, h6);
         auto comb = [&](int i, int j, int si, int sj) {
             const F2 sum = add2(fma2(f2(k2[i], k2[j]), two, f2(k1[i], k1[j])),
@@ -174,10 +175,18 @@ __device__ __forceinline__ void step_g(const S* y, const S& E, const S& L, const
 #pragma unroll
         for (int i = 0; i < 7; ++i) t[sgxa::sidx(i)] = y[sgxa::sidx(i)] + k3[i] * he;
         rhs_g7(t, E, L, a, M, k4);
-        const S h6 = he / S(T(6));
+        if constexpr (std::is_same_v<S, double>) {
+            S ks[7];
+            const S h6 = sixth(he);
+            sgxa::ksum7(k1, k2, k3, k4, ks);
 #pragma unroll
-        for (int i = 0; i < 7; ++i)
-            o[sgxa::sidx(i)] = y[sgxa::sidx(i)] + ((k1[i] + k2[i] * S(T(2))) + (k3[i] * S(T(2)) + k4[i])) * h6;
+            for (int i = 0; i < 7; ++i) o[sgxa::sidx(i)] = y[sgxa::sidx(i)] + ks[i] * h6;
+        } else {
+            const S h6 = he / S(T(6));
+#pragma unroll
+            for (int i = 0; i < 7; ++i)
+                o[sgxa::sidx(i)] = y[sgxa::sidx(i)] + ((k1[i] + k2[i] * S(T(2))) + (k3[i] * S(T(2)) + k4[i])) * h6;
+        }
     }
     const S n = S(T(1.5)) - S(T(0.5)) * (o[6] * o[6] + o[7] * o[7]);
     o[6] = o[6] * n;
@@ -554,7 +563,7 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // words); CK = kCkSparse in a thread-local array.  Launched with
 // kBackwardThreads threads a block.
 template <class T, bool SLAB, bool DUALJ, int CK>
-__global__ void __launch_bounds__(kBackwardThreads, 4)
+__global__ void __launch_bounds__(kBackwardThreads, sizeof(T) == 8 ? 2 : 4)
     diff_backward_kernel(DiffConst<T> k, DiffParamsT<T> p, DiffBufs<T> b, const float* __restrict__ gimg) {
     constexpr bool SHARED = CK == kCkDense;
     extern __shared__ __align__(16) unsigned char diff_seg_raw[];

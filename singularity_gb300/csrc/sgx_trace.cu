@@ -325,7 +325,8 @@ template <class T, int FL> struct KerrAdaptive {
                 return true;
             }
         }
-        h = DM<T>::fmin_(h, T(pass.h_max_frac) * y.r);
+        if constexpr (std::is_same_v<T, double>) h = pos_min(h, T(pass.h_max_frac) * y.r);
+        else h = DM<T>::fmin_(h, T(pass.h_max_frac) * y.r);
         const KAttempt<T> at = kerr_attempt<T, FORM>(y, k1, h, v, c);
         ++steps;
         bool accept;
@@ -342,6 +343,10 @@ template <class T, int FL> struct KerrAdaptive {
             const T e = error_norm_fast(y, at, pass.tol);
             accept = e <= DLIT(1.0);
             h = h * step_factor_fast(e);
+        } else if constexpr (std::is_same_v<T, double>) {
+            const T e = error_norm_pos(y, at, pass.tol);
+            accept = e <= DLIT(1.0);
+            h = h * step_factor_pos(e);
         } else {
             const T e = error_norm<T>(y, at, pass.tol);
             accept = e <= DLIT(1.0);
