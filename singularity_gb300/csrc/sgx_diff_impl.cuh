@@ -34,7 +34,16 @@ using namespace sgxd;
 // form's memory budget, everything else the sparse one.
 constexpr int kCkSparse = 64;
 constexpr int kCkDense = 10;
-constexpr int kBackwardThreads = 128;
+// Threads a block of the one-ray-a-thread kernels.  Blocks of 128 leave SMs
+// idle when there are few rays: 24,576 rays are 192 of them on 152 SMs, and an
+// SM with two runs twice as long as one with one.  One-warp blocks spread such
+// a launch evenly.  Where the line lies (128 against 32 threads, ms on one
+// GB300): forward FP32 65,536 rays 0.53 / 0.46, 131,072 rays 0.72 / 0.66,
+// 262,144 1.05 / 1.04, 524,288 1.73 / 1.73; FP64 65,536 rays 18.2 / 13.9, 131,072
+// 27.4 / 27.5; backward FP64 8,192 rays 13.1 / 12.4, 32,768 21.1 / 18.6, 65,536
+// 32.1 / 33.3; FP32 crossing model 8,192 rays 0.96 / 0.62, 49,152 1.2 / 1.1.
+constexpr int kThreads = 128, kSmallThreads = 32;
+constexpr std::uint64_t kSmallForward = 1u << 18, kSmallBackward = 1u << 16;  // fewer rays: one-warp blocks
 constexpr int kMaxCross = 8;  // crossings recorded per ray (crossing model)
 constexpr int NS = 8;         // state: r, theta, phi, p_r, p_theta, psi (swept angle), sin(theta), cos(theta)
 constexpr int NC = NS + 1;    // checkpoint: state and transmittance
@@ -560,16 +569,16 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // step to the camera, one checkpoint segment at a time.  CK = kCkDense keeps
 // the recomputed segment in dynamic shared memory, (CK + 1) * NC values a
 // thread laid out [slot][value][thread] (consecutive threads, consecutive
-// words); CK = kCkSparse in a thread-local array.  Launched with
-// kBackwardThreads threads a block.
-template <class T, bool SLAB, bool DUALJ, int CK>
-__global__ void __launch_bounds__(kBackwardThreads, sizeof(T) == 8 ? 2 : 4)
+// words); CK = kCkSparse in a thread-local array.  Launched with at most TH
+// threads a block, exactly TH where the segment is shared.
+template <class T, bool SLAB, bool DUALJ, int CK, int TH>
+__global__ void __launch_bounds__(TH, (sizeof(T) == 8 ? 256 : 512) / TH)
     diff_backward_kernel(DiffConst<T> k, DiffParamsT<T> p, DiffBufs<T> b, const float* __restrict__ gimg) {
     constexpr bool SHARED = CK == kCkDense;
     extern __shared__ __align__(16) unsigned char diff_seg_raw[];
     // value v of slot j of this thread's segment (shared form)
     T* const seg = reinterpret_cast<T*>(diff_seg_raw) + threadIdx.x;
-    auto at = [](int j, int v) { return (j * NC + v) * kBackwardThreads; };
+    auto at = [](int j, int v) { return (j * NC + v) * TH; };
     const std::uint64_t id = std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (id >= b.n) return;
     double* gout = b.grads;
@@ -926,16 +935,17 @@ cudaError_t run_forward(sgx_diff_state& st, float* img, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b.overflow, 0, 16, s);
     if (e != cudaSuccess) return e;
     offsets_kernel<T><<<(k.spp + 127) / 128, 128, 0, s>>>(k.spp, const_cast<T*>(b.ox), const_cast<T*>(b.oy));
-    const unsigned grid = unsigned((st.n + 127) / 128);
+    const int th = st.n < kSmallForward ? kSmallThreads : kThreads;
+    const unsigned grid = unsigned((st.n + th - 1) / th);
     const bool slab = st.o.model == SGX_DIFF_MODEL_SLAB;
     bool dense = false;
     if constexpr (sizeof(T) == 4) dense = st.ck == std::uint32_t(kCkDense);
     if constexpr (sizeof(T) == 4) {
-        if (dense && slab) diff_forward_kernel<T, true, kCkDense><<<grid, 128, 0, s>>>(k, p, b);
-        else if (dense) diff_forward_kernel<T, false, kCkDense><<<grid, 128, 0, s>>>(k, p, b);
+        if (dense && slab) diff_forward_kernel<T, true, kCkDense><<<grid, th, 0, s>>>(k, p, b);
+        else if (dense) diff_forward_kernel<T, false, kCkDense><<<grid, th, 0, s>>>(k, p, b);
     }
-    if (!dense && slab) diff_forward_kernel<T, true, kCkSparse><<<grid, 128, 0, s>>>(k, p, b);
-    else if (!dense) diff_forward_kernel<T, false, kCkSparse><<<grid, 128, 0, s>>>(k, p, b);
+    if (!dense && slab) diff_forward_kernel<T, true, kCkSparse><<<grid, th, 0, s>>>(k, p, b);
+    else if (!dense) diff_forward_kernel<T, false, kCkSparse><<<grid, th, 0, s>>>(k, p, b);
     const std::uint64_t npix = std::uint64_t(k.width) * k.height;
     diff_image_kernel<T><<<unsigned((npix + 255) / 256), 256, 0, s>>>(k, b, img);
     return cudaGetLastError();
@@ -946,26 +956,30 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
     const DiffConst<T> k = make_const<T>(st.u, st.o);
     const DiffParamsT<T> p{T(st.p.spin), T(st.p.incl), T(st.p.r_in), T(st.p.t_scale)};
     DiffBufs<T> b = carve_bufs<T>(st, k.spp);
-    const unsigned grid = unsigned((st.n + kBackwardThreads - 1) / kBackwardThreads);
     const bool slab = st.o.model == SGX_DIFF_MODEL_SLAB, dual = st.o.adjoint_form == SGX_DIFF_ADJOINT_DUAL;
+    const int th = st.n < kSmallBackward ? kSmallThreads : kThreads;
+    const unsigned grid = unsigned((st.n + th - 1) / th);
     bool dense = false;
     if constexpr (sizeof(T) == 4) {
-        // the dense checkpoints pair with the hand-derived reverse pass only
+        // the dense checkpoints pair with the hand-derived reverse pass only;
+        // their segments are laid out for the block size
         dense = st.ck == std::uint32_t(kCkDense);
         if (dense) {
-            const int smem = (kCkDense + 1) * NC * kBackwardThreads * int(sizeof(T));
-            auto* kern = slab ? diff_backward_kernel<T, true, false, kCkDense>
-                              : diff_backward_kernel<T, false, false, kCkDense>;
+            const int smem = (kCkDense + 1) * NC * th * int(sizeof(T));
+            auto* kern = th == kThreads ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kThreads>
+                                                : diff_backward_kernel<T, false, false, kCkDense, kThreads>)
+                                        : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads>
+                                                : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads>);
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
-            kern<<<grid, kBackwardThreads, smem, s>>>(k, p, b, gimg);
+            kern<<<grid, th, smem, s>>>(k, p, b, gimg);
         }
     }
     if (!dense) {
-        if (slab && !dual) diff_backward_kernel<T, true, false, kCkSparse><<<grid, kBackwardThreads, 0, s>>>(k, p, b, gimg);
-        else if (slab) diff_backward_kernel<T, true, true, kCkSparse><<<grid, kBackwardThreads, 0, s>>>(k, p, b, gimg);
-        else if (!dual) diff_backward_kernel<T, false, false, kCkSparse><<<grid, kBackwardThreads, 0, s>>>(k, p, b, gimg);
-        else diff_backward_kernel<T, false, true, kCkSparse><<<grid, kBackwardThreads, 0, s>>>(k, p, b, gimg);
+        if (slab && !dual) diff_backward_kernel<T, true, false, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
+        else if (slab) diff_backward_kernel<T, true, true, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
+        else if (!dual) diff_backward_kernel<T, false, false, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
+        else diff_backward_kernel<T, false, true, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
     }
     const std::uint32_t nchunks = std::uint32_t((st.n + 1023) / 1024);
     double* part = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(b.overflow) + 256);
