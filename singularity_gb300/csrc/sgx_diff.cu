@@ -20,11 +20,13 @@
 // Adjoint: given dLoss/dImage, each ray seeds dLoss/dhdr and sweeps the steps
 // backwards from its last emitting step, one checkpoint segment at a time
 // (the segment's states recomputed from its checkpoint into shared memory
-// for 10-step segments, thread-local memory for 64-step ones).  Emission terms go through the transmittance chain with their
-// local derivatives from dual numbers (sgx_dual.cuh); the adjoint vector is
-// carried through each RK4 step by the hand-derived reverse pass of
-// sgx_adjoint.cuh (or, as a cross-check, by the step's Jacobian built with
-// dual numbers); the camera set-up is differentiated with dual numbers.
+// for 10-step segments, thread-local memory for 64-step ones).  Emission terms
+// go through the transmittance chain with local derivatives from hand-derived
+// reverse passes of the colour and the absorption (the crossing model's formed
+// before the sweep from the states the forward stored at each crossing); the
+// adjoint vector is carried through each RK4 step by the reverse pass of
+// sgx_adjoint.cuh.  As a cross-check both can be built with dual numbers
+// (sgx_dual.cuh) instead; the camera set-up is always differentiated so.
 // Per-ray gradients are summed in a fixed order, so the result is
 // deterministic.
 
@@ -114,13 +116,15 @@ sgx_status sgx_diff_forward(sgx_context* c, const sgx_uniforms* base, const sgx_
     if (need > limit)
         return fail(c, SGX_ERR_INVALID_ARGUMENT, "differentiable render needs " + std::to_string(need >> 20) +
                                                      " MiB of records: fewer rays or max_steps");
-    if (st.cap < need) {
+    const std::size_t all = need + (o.precision == SGX_PRECISION_FP64 ? crossing_bytes<double>(st.n, st.nx)
+                                                                      : crossing_bytes<float>(st.n, st.nx));
+    if (st.cap < all) {
         if (st.mem) cudaFree(st.mem);
         st.mem = nullptr;
         st.cap = 0;
-        cudaError_t e = cudaMalloc(&st.mem, need);
+        cudaError_t e = cudaMalloc(&st.mem, all);
         if (e != cudaSuccess) return cuda_fail(c, e, "sgx_diff_forward: cudaMalloc");
-        st.cap = need;
+        st.cap = all;
     }
     const std::size_t img_bytes = std::size_t(base->width) * base->height * 3 * sizeof(float);
     if (d_image == nullptr) {
