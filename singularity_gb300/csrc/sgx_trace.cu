@@ -346,7 +346,9 @@ template <class T, int FL> struct KerrAdaptive {
         }
         if (in_zone) {
             ++zone;
-            const double e = error_norm_fp64_1div(y, at, pass.tol);
+            double e;
+            if constexpr (FAST && std::is_same_v<T, float>) e = error_norm_zone(y, at, pass.tol);
+            else e = error_norm_fp64_1div(y, at, pass.tol);
             accept = e <= 1.0;
             h = h * step_factor_fast(float(e));
         } else if constexpr (FAST && std::is_same_v<T, float>) {

@@ -1,8 +1,9 @@
 // Test program (built and run by tests/test_gpu_division.py): the arithmetic of
 // sgx_device.cuh that stands for divisions and square roots, against the
 // compiler's own, and one step of the FP32 fixed-step forms with shared
-// reciprocals against the same step with compiled divisions.  Prints mismatch
-// counts (FP32: bit for bit) and worst errors in units of the last place (FP64).
+// reciprocals against the same step with compiled divisions, and the precision
+// form's error norm from one component.  Prints mismatch counts
+// (FP32: bit for bit) and worst errors in units of the last place (FP64).
 #include <cmath>
 #include <cstdio>
 
@@ -10,7 +11,7 @@
 
 using namespace sgxd;
 
-__device__ unsigned long long g_bad[6];
+__device__ unsigned long long g_bad[7];
 __device__ unsigned long long g_ulp[2];
 
 __device__ __forceinline__ std::uint32_t mix(std::uint32_t x) {
@@ -101,14 +102,49 @@ __global__ void steps() {
         atomicAdd(&g_bad[5], 1ull);
 }
 
+// The precision form's error norm from one FP64 component against the norm over
+// all of them: random attempts, with ties, near ties, zeros and NaN among the
+// components.
+__global__ void norms() {
+    std::uint32_t s = mix(blockIdx.x * blockDim.x + threadIdx.x + 77u);
+    auto uni = [&]() {
+        s = mix(s + 0x9e3779b9u);
+        return float(s >> 8) * 0x1p-24f;
+    };
+    float y[6], y4[6], k4[6], k5[6];
+    const float tie = uni(), d0 = exp2f(-30.0f * uni());
+    for (int i = 0; i < 6; ++i) {
+        y[i] = exp2f(10.0f * uni() - 8.0f) * (uni() < 0.5f ? -1.0f : 1.0f);
+        y4[i] = y[i] * (1.0f + 0.01f * uni());
+        k4[i] = uni() - 0.5f;
+        float d = exp2f(-30.0f * uni());
+        if (tie < 0.3f) {  // ratios equal to a few ulp
+            y[i] = y[0];
+            y4[i] = y4[0];
+            d = d0 * (1.0f + 0x1p-22f * float(int(8.0f * uni())));
+            k4[i] = 1.0f;
+        }
+        k5[i] = k4[i] - d;
+        if (tie > 0.95f && uni() < 0.3f) k5[i] = k4[i];
+        if (tie > 0.99f && uni() < 0.3f) k5[i] = NAN;
+    }
+    auto six = [](const float* v) { return KSC<float>{v[0], v[1], v[2], v[3], v[4], v[5]}; };
+    const KSC<float> Y = six(y);
+    const KAttempt<float> A{six(y4), six(k4), six(k5), exp2f(-8.0f * uni())};
+    const double one = error_norm_zone(Y, A, 1e-6f), all = error_norm_fp64_1div(Y, A, 1e-6f);
+    if (__double_as_longlong(one) != __double_as_longlong(all)) atomicAdd(&g_bad[6], 1ull);
+}
+
 int main() {
     for (int e : {-60, -20, -3, -1, 0, 1, 2, 9, 28, 60}) single<<<(1 << 23) / 256, 256>>>(e, -30, 30);
     for (int e : {-67, -20, -1, 0, 1, 7, 16, 40}) dbl<<<(1 << 23) / 256, 256>>>(e);
     steps<<<(1 << 22) / 256, 256>>>();
-    unsigned long long bad[6], ulp[2];
+    norms<<<(1 << 22) / 256, 256>>>();
+    unsigned long long bad[7], ulp[2];
     cudaMemcpyFromSymbol(bad, g_bad, sizeof(bad));
     cudaMemcpyFromSymbol(ulp, g_ulp, sizeof(ulp));
     if (cudaDeviceSynchronize() != cudaSuccess) return 1;
-    std::printf("%llu %llu %llu %llu %llu %llu %llu %llu\n", bad[0], bad[1], bad[2], bad[3], bad[4], bad[5], ulp[0], ulp[1]);
+    std::printf("%llu %llu %llu %llu %llu %llu %llu %llu %llu\n", bad[0], bad[1], bad[2], bad[3], bad[4], bad[5], bad[6], ulp[0],
+                ulp[1]);
     return 0;
 }

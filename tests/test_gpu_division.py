@@ -3,7 +3,8 @@
 FP32: the shared-reciprocal quotients, the reciprocal behind them and x / 6
 give the correctly rounded result, so they equal the compiled division bit for
 bit, for every significand of the divisor, and a fixed step that divides so
-equals one with compiled divisions, whatever the state.  FP64: the Newton reciprocal is
+equals one with compiled divisions, whatever the state.  The precision form's
+norm from one component is the norm over all six, bit for bit.  FP64: the Newton reciprocal is
 rounded twice (its correction and the sum), the square root likewise: within
 1 ulp of the rounded result.
 """
@@ -26,8 +27,8 @@ def test_divisions_match_the_compilers(tmp_path, sgx):
     subprocess.run([B._nvcc(), *B.ARCH, *B.NVCC_FLAGS, str(ROOT / "tests" / "division_check.cu"), "-o", str(exe)],
                    check=True, capture_output=True, text=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout
-    reciprocal, sixth, quotient, edge, kerr, schwarzschild, rcp_ulp, sqrt_ulp = map(int, out.split())
+    reciprocal, sixth, quotient, edge, kerr, schwarzschild, norm, rcp_ulp, sqrt_ulp = map(int, out.split())
     print(out)
     assert reciprocal == sixth == quotient == edge == 0
-    assert kerr == schwarzschild == 0
+    assert kerr == schwarzschild == norm == 0
     assert rcp_ulp <= 1 and sqrt_ulp <= 1
