@@ -176,14 +176,16 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
     if (s != SGX_OK) return s;
 
     SGX_CUDA(c, cudaMemcpyAsync(c->d_u, u, sizeof(sgx_uniforms), cudaMemcpyHostToDevice, st));
-    SGX_CUDA(c, sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), st));
+    SGX_CUDA(c, sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), o.tolerance, st));
     // The tracer takes the view's constants as a kernel parameter: a host copy
     // of the device-computed slot, refreshed when the uniforms change.
-    if (c->h_view_precision != int(o.precision) || std::memcmp(&c->h_view_u, u, sizeof(sgx_uniforms)) != 0) {
+    if (c->h_view_precision != int(o.precision) || c->h_view_tol != o.tolerance ||
+        std::memcmp(&c->h_view_u, u, sizeof(sgx_uniforms)) != 0) {
         c->h_view_precision = -1;
         SGX_CUDA(c, cudaMemcpyAsync(c->h_view, c->d_view, sgxk::view_bytes(), cudaMemcpyDeviceToHost, st));
         SGX_CUDA(c, cudaStreamSynchronize(st));
         c->h_view_u = *u;
+        c->h_view_tol = o.tolerance;
         c->h_view_precision = int(o.precision);
     }
     const std::uint32_t tw = o.tile_w;
@@ -460,7 +462,7 @@ sgx_status sgx_trace_samples(sgx_context* c, const sgx_uniforms* u, const sgx_re
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_gy, gy, n * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_s, s, n * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_u, u, sizeof(sgx_uniforms), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), c->stream);
+    if (e == cudaSuccess) e = sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), o.tolerance, c->stream);
     if (e == cudaSuccess)
         e = sgxk::launch_probe(c->d_view, int(u->metric_type), int(o.precision), int(o.integrator), int(o.rhs_form), n, d_gx,
                                d_gy, d_s, d_hdr, d_steps, d_term, probe_opts(o), c->stream);
@@ -517,7 +519,7 @@ sgx_status sgx_trace_invariants(sgx_context* c, const sgx_uniforms* u, const sgx
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_gy, gy, n * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_s, s, n * 4, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_u, u, sizeof(sgx_uniforms), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), c->stream);
+    if (e == cudaSuccess) e = sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), o.tolerance, c->stream);
     if (e == cudaSuccess)
         e = sgxk::launch_invariants(c->d_view, int(o.precision), int(o.rhs_form), n, d_gx, d_gy, d_s, d_inv, d_term,
                                     probe_opts(o), c->stream);

@@ -69,7 +69,7 @@ cudaError_t enqueue(sgx_batch* b, const sgx_render_opts& o, const sgxk::ViewPlan
     pass.zone = o.fp64_zone;
     pass.project = o.projection;
     cudaError_t e = cudaMemsetAsync(b->d_counters, 0, sizeof(sgxk::PassCounters), st);
-    if (e == cudaSuccess) e = sgxk::launch_setup_views(b->d_u, b->n, b->d_views, int(o.precision), st);
+    if (e == cudaSuccess) e = sgxk::launch_setup_views(b->d_u, b->n, b->d_views, int(o.precision), o.tolerance, st);
     if (e == cudaSuccess)
         e = sgxk::launch_trace(int(b->metric), int(o.precision), int(o.integrator), int(o.rhs_form), pass,
                                sgxk::LaunchShape{int(o.block_threads), int(o.blocks_per_sm)}, st);

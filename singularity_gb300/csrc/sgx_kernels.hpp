@@ -122,7 +122,7 @@ ViewSet make_view_set(const ViewPlan& plan, const void* d_views, const std::uint
 
 // Per-view constants (device) from device copies of the uniforms, one thread each.
 cudaError_t launch_setup_views(const sgx_uniforms* d_u, std::uint32_t n, void* d_views, int precision,
-                               cudaStream_t st);
+                               float tol, cudaStream_t st);
 
 // Persistent tracer over a ViewSet.  precision: sgx_precision; integrator: sgx_integrator.
 // h_view: for a single-view pass, a host copy of that view's constants

@@ -190,7 +190,7 @@ extern "C" sgx_status sgx_render_noalloc(const sgx_uniforms* u, const sgx_render
     e = cudaMemcpyAsync(d_u, u, sizeof(sgx_uniforms), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_words, plan.words, plan.word_count * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(sgxk::PassCounters), st);
-    if (e == cudaSuccess) e = sgxk::launch_setup_views(d_u, 1, d_view, int(o.precision), st);
+    if (e == cudaSuccess) e = sgxk::launch_setup_views(d_u, 1, d_view, int(o.precision), o.tolerance, st);
     if (e == cudaSuccess)
         e = sgxk::launch_trace(int(u->metric_type), int(o.precision), int(o.integrator), int(o.rhs_form), pass,
                                shape, st);

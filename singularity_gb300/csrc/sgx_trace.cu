@@ -352,7 +352,7 @@ template <class T, int FL> struct KerrAdaptive {
             accept = e <= 1.0;
             h = h * step_factor_fast(float(e));
         } else if constexpr (FAST && std::is_same_v<T, float>) {
-            const T e = error_norm_fast(y, at, pass.tol);
+            const T e = error_norm_fast(y, at, v.inv_tol);
             accept = e <= DLIT(1.0);
             h = h * step_factor_fast(e);
         } else if constexpr (std::is_same_v<T, double>) {
@@ -712,9 +712,9 @@ __global__ void __launch_bounds__(128) trace_invariants(const View<T>* __restric
     if (term != nullptr) term[i] = ray.term;
 }
 
-template <class T> __global__ void setup_views(const sgx_uniforms* u, std::uint32_t n, View<T>* out) {
+template <class T> __global__ void setup_views(const sgx_uniforms* u, std::uint32_t n, View<T>* out, float tol) {
     const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = make_view<T>(u[i]);
+    if (i < n) out[i] = make_view<T>(u[i], tol);
 }
 
 // Final encode of a pixel's mean (geodesic_kernel.cu:502-509).
@@ -1037,13 +1037,13 @@ ViewSet make_view_set(const ViewPlan& plan, const void* d_views, const std::uint
 }
 
 cudaError_t launch_setup_views(const sgx_uniforms* d_u, std::uint32_t n, void* d_views, int precision,
-                               cudaStream_t st) {
+                               float tol, cudaStream_t st) {
     const unsigned threads = 64;
     const unsigned blocks = (n + threads - 1) / threads;
     if (precision == SGX_PRECISION_FP64) {
-        setup_views<double><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<double>*>(d_views));
+        setup_views<double><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<double>*>(d_views), tol);
     } else {
-        setup_views<float><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<float>*>(d_views));
+        setup_views<float><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<float>*>(d_views), tol);
     }
     return cudaGetLastError();
 }
