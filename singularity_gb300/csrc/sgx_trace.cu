@@ -86,8 +86,11 @@ constexpr int FL_DIV = 32;
 
 // Kerr, fixed step (geodesic_kernel.cu:303-403).
 template <class T, int FL> struct KerrFixed {
-    static constexpr int kMinBlocks = sizeof(T) == 4 ? 4 : 1;
-    static constexpr int kMinBlocksMulti = kMinBlocks;
+    // 56 registers (36 warps an SM): 1080p x 16 44.8 -> 44.3 ms, the reference
+    // form 1279 x 719 x 4 12.9 -> 12.6 ms; 48 spill (47.1, 14.5 ms)
+    static constexpr int kRegs = sizeof(T) == 4 ? ((FL & FL_SC) ? 64 : 56) : 255;
+    static constexpr int kRegsMulti = sizeof(T) == 4 ? 64 : 255;
+    static constexpr bool kCountDown = false;
     static constexpr bool FAST = (FL & FL_FAST) != 0;
     static constexpr bool SC = (FL & FL_SC) != 0;
     static constexpr int FORM = FAST ? RHS_SEP : RHS_REF;
@@ -166,8 +169,8 @@ template <class T, int FL> struct KerrFixed {
 
 // Schwarzschild, fixed step (geodesic_kernel.cu:229-297).
 template <class T, int FL> struct SchwFixed {
-    static constexpr int kMinBlocks = sizeof(T) == 4 ? 4 : 1;
-    static constexpr int kMinBlocksMulti = kMinBlocks;
+    static constexpr int kRegs = sizeof(T) == 4 ? 64 : 255, kRegsMulti = kRegs;
+    static constexpr bool kCountDown = false;
     SS<T> y;
     T prev_th, prev_r, prev_uph;
     T t0, t1, t2;
@@ -234,11 +237,16 @@ template <class T, int FL> struct KerrAdaptive {
     static constexpr bool MIXED = (FL & FL_MIXED) != 0;
     static constexpr bool RTPROJ = (FL & FL_RTPROJ) != 0;
     static constexpr bool RANGE = (FL & FL_RANGE) != 0;
-    static constexpr int kMinBlocks = sizeof(T) == 4 ? 4 : 1;
-    // Multi-view passes hold their view's constants in shared memory and
-    // registers rather than the constant bank: 80 registers (3 blocks) beat
-    // 64 with spills there (1954 against 1877 Mrays/s on six 4K views).
-    static constexpr int kMinBlocksMulti = sizeof(T) == 4 ? 3 : 1;
+    // 64 registers with up to 60 bytes of spills beat 56 and 72 (1080p x 16 mixed
+    // 11.65 ms against 12.1 and, by one block less, 11.9).  Multi-view passes
+    // hold their view's constants in shared memory and registers rather than the
+    // constant bank: FP32 72 registers without spills (28 warps; 74 leave 24),
+    // the others 80.
+    static constexpr int kRegs = sizeof(T) == 4 ? 64 : 255;
+    static constexpr int kRegsMulti = sizeof(T) == 4 ? (FAST && !MIXED ? 72 : 80) : 255;
+    // counting the steps left down suits this kernel's register allocation: 64
+    // batched views 185.4 -> 182.6 ms; the others run 1-5 % slower with it
+    static constexpr bool kCountDown = RANGE && FAST && !MIXED && sizeof(T) == 4;
     KSC<T> y, k1;  // theta carried as (sin theta, cos theta)
     KC<T> c;
     T Q;           // Carter constant the projection holds p_theta to
@@ -412,9 +420,18 @@ template <class T, int FL> struct KerrAdaptive {
 // 256 x 256 7.23 -> 6.96 ms; the frames are the same bit for bit.
 template <class T, class Ray>
 __device__ __forceinline__ bool run_ray(Ray& ray, const View<T>& v, const PassDesc& pass, std::uint32_t stop) {
-    do {
-        if (ray.step(v, pass)) return true;
-    } while (ray.steps < stop);
+    if constexpr (Ray::kCountDown) {  // the other shape of the same loop (KerrAdaptive::kCountDown)
+        std::uint32_t left = stop - ray.steps;
+        bool end = false;
+        do {
+            end = ray.step(v, pass);
+        } while (!end && --left != 0u);
+        if (end) return true;
+    } else {
+        do {
+            if (ray.step(v, pass)) return true;
+        } while (ray.steps < stop);
+    }
     if (stop < v.max_steps) return false;
     ray.term = TERM_BUDGET;
     return true;
@@ -524,15 +541,14 @@ enum : int { MODE_IDLE = 0, MODE_ACTIVE = 1, MODE_DONE = 2 };
 // The persistent tracer over a set of views.  Ray ids enumerate, view by
 // view, tiles of tile_w x tile_h pixels (padded to whole tiles), the pixels
 // of a tile row-major, and a pixel's samples innermost; ids that land in the
-// padding carry no work.  Each policy names its resident blocks of 256 per
-// SM (kMinBlocks for a single view, kMinBlocksMulti for a batch), which caps
-// its registers: 4 = 64 registers, 3 = 80; FP64 variants keep their
-// registers (capped they spill up to 1.4 KB).
+// padding carry no work.  Each policy names its registers a thread (kRegs for
+// a single view, kRegsMulti for a batch); blocks are at most 256 threads.  FP64
+// variants keep theirs (capped they spill up to 1.4 KB).
 // ONE: a single-view pass whose constants arrive as the kernel parameter
 // `one`, read from the constant bank as instruction operands instead of
 // shared-memory loads held in registers.
 template <class T, class Ray, bool ONE>
-__global__ void __launch_bounds__(256, ONE ? Ray::kMinBlocks : Ray::kMinBlocksMulti)
+__global__ void __maxnreg__(ONE ? Ray::kRegs : Ray::kRegsMulti)
     trace_persistent(const __grid_constant__ PassDesc pass, const __grid_constant__ View<T> one) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // Block totals of the ray counters and each lane's record slot live in
