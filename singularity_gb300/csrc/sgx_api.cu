@@ -147,6 +147,9 @@ sgxk::PassDesc probe_opts(const sgx_render_opts& o) {
     return p;
 }
 
+// Layout words of one view, behind the uniform block.
+constexpr std::size_t kUniformWords = 6;
+
 std::uint32_t clamp_spp(std::uint32_t ss) { return ss < 1u ? 1u : (ss > 1024u ? 1024u : ss); }
 
 // One render (all passes of [begin, begin+count)) into `out` with `format`.
@@ -165,29 +168,22 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
     if (rows == 0u) return fail(c, SGX_ERR_INVALID_ARGUMENT, "the frame slice has no rows");
     const std::uint32_t npix = u->width * rows;
 
-    // Pass size under the workspace budget.
-    std::size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    std::size_t budget = std::min(c->workspace_budget, free_b / 2 + c->results_cap);
-    std::uint64_t per_sample = std::uint64_t(npix) * sgxk::record_bytes(int(o.precision));
-    std::uint32_t S = std::uint32_t(std::max<std::uint64_t>(1, std::min<std::uint64_t>(count, budget / per_sample)));
-    S = std::min(S, sgxk::kMaxPassSamplesHost);
-    sgx_status s = ensure_results(c, std::size_t(S) * per_sample);
-    if (s != SGX_OK) return s;
-
-    SGX_CUDA(c, cudaMemcpyAsync(c->d_u, u, sizeof(sgx_uniforms), cudaMemcpyHostToDevice, st));
-    SGX_CUDA(c, sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), o.tolerance, st));
-    // The tracer takes the view's constants as a kernel parameter: a host copy
-    // of the device-computed slot, refreshed when the uniforms change.
-    if (c->h_view_precision != int(o.precision) || c->h_view_tol != o.tolerance ||
-        std::memcmp(&c->h_view_u, u, sizeof(sgx_uniforms)) != 0) {
-        c->h_view_precision = -1;
-        SGX_CUDA(c, cudaMemcpyAsync(c->h_view, c->d_view, sgxk::view_bytes(), cudaMemcpyDeviceToHost, st));
-        SGX_CUDA(c, cudaStreamSynchronize(st));
-        c->h_view_u = *u;
-        c->h_view_tol = o.tolerance;
-        c->h_view_precision = int(o.precision);
+    // Pass size under the workspace budget.  The free memory is asked for only
+    // when the record buffer has to grow (the query takes longer than the rest
+    // of a small frame's set-up).
+    const std::uint64_t per_sample = std::uint64_t(npix) * sgxk::record_bytes(int(o.precision));
+    auto samples_in = [&](std::size_t budget) {
+        const std::uint64_t n = std::max<std::uint64_t>(1, std::min<std::uint64_t>(count, budget / per_sample));
+        return std::min(std::uint32_t(n), sgxk::kMaxPassSamplesHost);
+    };
+    std::uint32_t S = samples_in(c->workspace_budget);
+    if (std::size_t(S) * per_sample > c->results_cap) {
+        std::size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        S = samples_in(std::min(c->workspace_budget, free_b / 2 + c->results_cap));
     }
+    const sgx_status s = ensure_results(c, std::size_t(S) * per_sample);
+    if (s != SGX_OK) return s;
     const std::uint32_t tw = o.tile_w;
     const std::uint32_t th = o.tile_h;
     // An HDR frame into the context's image fuses the bloom extract into its
@@ -208,15 +204,44 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
     }
 
     sgx_render_stats acc{};
+    std::uint64_t* const d_words = reinterpret_cast<std::uint64_t*>(c->d_u + 1);
     for (std::uint32_t done = 0; done < count;) {
         const std::uint32_t n = std::min(S, count - done);
         const std::uint32_t s0 = begin + done;
         sgxk::ViewPlan plan;
         if (!sgxk::plan_views(u, 1, s0, n, tw, th, plan, slice))
             return fail(c, SGX_ERR_INVALID_ARGUMENT, "invalid pass or tile shape");
-        SGX_CUDA(c, cudaMemcpyAsync(c->d_words, plan.words, plan.word_count * 8, cudaMemcpyHostToDevice, st));
+        if (done == 0) {
+            // One copy brings the uniforms and the first pass's layout words
+            // (they follow the uniform block); the view's set-up clears the
+            // counters.  The tracer takes the view's constants as a kernel
+            // parameter: the set-up kernel also writes them to pinned host
+            // memory when the uniforms have changed.
+            struct {
+                sgx_uniforms u;
+                std::uint64_t words[kUniformWords];
+            } up;
+            static_assert(sizeof(up) == sizeof(sgx_uniforms) + 8 * kUniformWords, "copied as one block");
+            up.u = *u;
+            std::memcpy(up.words, plan.words, plan.word_count * 8);
+            const bool cached = c->h_view_precision == int(o.precision) && c->h_view_tol == o.tolerance &&
+                                std::memcmp(&c->h_view_u, u, sizeof(sgx_uniforms)) == 0;
+            if (!cached) c->h_view_precision = -1;
+            SGX_CUDA(c, cudaMemcpyAsync(c->d_u, &up, sizeof(up), cudaMemcpyHostToDevice, st));
+            SGX_CUDA(c, sgxk::launch_setup_views(c->d_u, 1, c->d_view, int(o.precision), o.tolerance, st, c->d_counters,
+                                                 cached ? nullptr : c->h_view));
+            if (!cached) {
+                SGX_CUDA(c, cudaStreamSynchronize(st));
+                c->h_view_u = *u;
+                c->h_view_tol = o.tolerance;
+                c->h_view_precision = int(o.precision);
+            }
+        } else {
+            SGX_CUDA(c, cudaMemcpyAsync(d_words, plan.words, plan.word_count * 8, cudaMemcpyHostToDevice, st));
+            SGX_CUDA(c, cudaMemsetAsync(c->d_counters, 0, sizeof(sgxk::PassCounters), st));
+        }
         sgxk::PassDesc pass{};
-        pass.vs = sgxk::make_view_set(plan, c->d_view, c->d_words);
+        pass.vs = sgxk::make_view_set(plan, c->d_view, d_words);
         pass.refill = o.refill_interval == 0 ? sgxk::kDefaultRefill : o.refill_interval;
         pass.results = c->d_results;
         pass.counters = c->d_counters;
@@ -225,8 +250,6 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
         pass.h_max_frac = o.h_max_frac;
         pass.zone = o.fp64_zone;
         pass.project = o.projection;
-        SGX_CUDA(c, cudaEventRecord(c->ev_begin, st));
-        SGX_CUDA(c, cudaMemsetAsync(c->d_counters, 0, sizeof(sgxk::PassCounters), st));
         SGX_CUDA(c, cudaEventRecord(c->ev_trace0, st));
         sgxk::LaunchShape shape{int(o.block_threads), int(o.blocks_per_sm)};
         SGX_CUDA(c, sgxk::launch_trace(int(u->metric_type), int(o.precision), int(o.integrator), int(o.rhs_form),
@@ -234,15 +257,15 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
         SGX_CUDA(c, cudaEventRecord(c->ev_trace1, st));
         const bool first = (s0 == 0);
         const bool finalize = (s0 + n == spp);
+        // the accumulation also writes the pass's counters to pinned host memory
+        const sgxk::CounterReport report{c->d_counters, c->h_counters};
         if (finalize && fuse_ext)
             SGX_CUDA(c, sgxk::launch_accumulate_hdr_extract(int(o.precision), pass.vs, c->d_results, c->d_acc, first,
                                                             out, c->d_bloom, u->width, u->height,
-                                                            u->bloom_threshold, st));
+                                                            u->bloom_threshold, st, report));
         else
             SGX_CUDA(c, sgxk::launch_accumulate(int(o.precision), pass.vs, c->d_results, c->d_acc, first, finalize,
-                                                format, out, st));
-        SGX_CUDA(c, cudaMemcpyAsync(c->h_counters, c->d_counters, sizeof(sgxk::PassCounters),
-                                    cudaMemcpyDeviceToHost, st));
+                                                format, out, st, report));
         SGX_CUDA(c, cudaEventRecord(c->ev_end, st));
         SGX_CUDA(c, cudaEventSynchronize(c->ev_end));
         acc.rays += c->h_counters->rays;
@@ -251,7 +274,7 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
         acc.zone_steps += c->h_counters->zone_steps;
         acc.budget_hits += c->h_counters->budget_hits;
         cudaEventElapsedTime(&acc.trace_ms, c->ev_trace0, c->ev_trace1);
-        cudaEventElapsedTime(&acc.total_ms, c->ev_begin, c->ev_end);
+        cudaEventElapsedTime(&acc.total_ms, c->ev_trace0, c->ev_end);
         done += n;
         c->next_sample = s0 + n;
         if (own) c->frame_valid = finalize;
@@ -321,13 +344,11 @@ sgx_status sgx_create(int device, sgx_context** out) {
     c->device = device;
     bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&c->d_view, sgxk::view_bytes() * sgxk::kMaxLaunchViews) == cudaSuccess;
-    ok = ok && cudaMalloc(reinterpret_cast<void**>(&c->d_u), sizeof(sgx_uniforms) * sgxk::kMaxLaunchViews) ==
-                   cudaSuccess;
-    ok = ok && cudaMalloc(reinterpret_cast<void**>(&c->d_words), sizeof(sgxk::ViewPlan::words)) == cudaSuccess;
+    ok = ok && cudaMalloc(reinterpret_cast<void**>(&c->d_u), sizeof(sgx_uniforms) + 8 * kUniformWords) == cudaSuccess;
     ok = ok && cudaMalloc(reinterpret_cast<void**>(&c->d_counters), sizeof(sgxk::PassCounters)) == cudaSuccess;
     ok = ok && cudaMallocHost(reinterpret_cast<void**>(&c->h_counters), sizeof(sgxk::PassCounters)) == cudaSuccess;
     ok = ok && cudaMallocHost(&c->h_view, sgxk::view_bytes()) == cudaSuccess;
-    ok = ok && cudaEventCreate(&c->ev_begin) == cudaSuccess && cudaEventCreate(&c->ev_trace0) == cudaSuccess
+    ok = ok && cudaEventCreate(&c->ev_trace0) == cudaSuccess
          && cudaEventCreate(&c->ev_trace1) == cudaSuccess && cudaEventCreate(&c->ev_end) == cudaSuccess;
     if (!ok) {
         sgx_destroy(c);
@@ -345,11 +366,10 @@ void sgx_destroy(sgx_context* c) {
     sgx_internal_free_diff(c);
     if (c->d_view) cudaFree(c->d_view);
     if (c->d_u) cudaFree(c->d_u);
-    if (c->d_words) cudaFree(c->d_words);
     if (c->d_counters) cudaFree(c->d_counters);
     if (c->h_counters) cudaFreeHost(c->h_counters);
     if (c->h_view) cudaFreeHost(c->h_view);
-    for (cudaEvent_t ev : {c->ev_begin, c->ev_trace0, c->ev_trace1, c->ev_end})
+    for (cudaEvent_t ev : {c->ev_trace0, c->ev_trace1, c->ev_end})
         if (ev) cudaEventDestroy(ev);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;

@@ -24,15 +24,14 @@ struct sgx_context {
     void* d_results = nullptr;     // results_cap bytes (hit records)
     std::size_t results_cap = 0;
     void* d_view = nullptr;            // kMaxLaunchViews view slots
-    sgx_uniforms* d_u = nullptr;       // kMaxLaunchViews uniform blocks
-    std::uint64_t* d_words = nullptr;  // view-set layout words
+    sgx_uniforms* d_u = nullptr;       // uniform block, and a pass's view-set layout words behind it
     sgxk::PassCounters* d_counters = nullptr;
     sgxk::PassCounters* h_counters = nullptr;  // pinned
     void* h_view = nullptr;            // pinned host copy of view slot 0 (single-view tracer parameter)
     sgx_uniforms h_view_u{};           // ... made from these uniforms
     float h_view_tol = 0.0f;           // ... and tolerance ...
     int h_view_precision = -1;         // ... at this precision (-1: none yet)
-    cudaEvent_t ev_begin = nullptr, ev_trace0 = nullptr, ev_trace1 = nullptr, ev_end = nullptr;
+    cudaEvent_t ev_trace0 = nullptr, ev_trace1 = nullptr, ev_end = nullptr;
     bool frame_valid = false;     // accumulator holds a complete frame
     std::uint32_t frame_spp = 0;
     std::uint32_t frame_format = SGX_FORMAT_RGBA8_SRGB;

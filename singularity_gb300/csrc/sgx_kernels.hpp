@@ -98,6 +98,13 @@ struct LaunchShape {
     int blocks_per_sm;
 };
 
+// Counters of a finished pass and the pinned host copy an accumulation makes of
+// them (host = nullptr: none).
+struct CounterReport {
+    const PassCounters* counters = nullptr;
+    PassCounters* host = nullptr;
+};
+
 // Host plan of a ViewSet: the layout block's contents (to copy to the device
 // as one array of 64-bit words) and the totals.  S_pass == 0 -> every view's
 // own samples per pixel.
@@ -120,9 +127,11 @@ bool plan_views(const sgx_uniforms* u, std::uint32_t n, std::uint32_t s0, std::u
 // the views at d_views.
 ViewSet make_view_set(const ViewPlan& plan, const void* d_views, const std::uint64_t* d_words);
 
-// Per-view constants (device) from device copies of the uniforms, one thread each.
+// Per-view constants (device) from device copies of the uniforms, one thread
+// each; when given, clears counters and writes the first view to host (pinned,
+// view_bytes()) too.
 cudaError_t launch_setup_views(const sgx_uniforms* d_u, std::uint32_t n, void* d_views, int precision,
-                               float tol, cudaStream_t st);
+                               float tol, cudaStream_t st, PassCounters* counters = nullptr, void* host = nullptr);
 
 // Persistent tracer over a ViewSet.  precision: sgx_precision; integrator: sgx_integrator.
 // h_view: for a single-view pass, a host copy of that view's constants
@@ -149,7 +158,8 @@ cudaError_t launch_invariants(const void* d_view, int precision, int rhs_form, s
 // per pixel, packed over views); when `finalize`, also writes every view's
 // frame in `format` to out (packed like acc; scale 1/spp of each view).
 cudaError_t launch_accumulate(int precision, const ViewSet& vs, const void* results, float4* acc, bool first,
-                              bool finalize, std::uint32_t format, void* out, cudaStream_t st);
+                              bool finalize, std::uint32_t format, void* out, cudaStream_t st,
+                              CounterReport report = {});
 
 // The last pass of a single-view, unsliced SGX_FORMAT_RGBA16F_HDR frame (W x
 // H, W and H >= 2) with the bloom extract fused in: as launch_accumulate with
@@ -157,7 +167,7 @@ cudaError_t launch_accumulate(int precision, const ViewSet& vs, const void* resu
 // extract of each 2x2 block of the half-precision frame at `threshold`.
 cudaError_t launch_accumulate_hdr_extract(int precision, const ViewSet& vs, const void* results, float4* acc,
                                           bool first, void* out, void* ext, std::uint32_t W, std::uint32_t H,
-                                          float threshold, cudaStream_t st);
+                                          float threshold, cudaStream_t st, CounterReport report = {});
 
 // Re-encodes an accumulated single-view frame (acc, float4 mean-sum) in another format.
 cudaError_t launch_encode(const float4* acc, std::uint32_t npix, float scale, std::uint32_t format, void* out,

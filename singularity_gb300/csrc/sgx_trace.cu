@@ -728,9 +728,16 @@ __global__ void __launch_bounds__(128) trace_invariants(const View<T>* __restric
     if (term != nullptr) term[i] = ray.term;
 }
 
-template <class T> __global__ void setup_views(const sgx_uniforms* u, std::uint32_t n, View<T>* out, float tol) {
+template <class T>
+__global__ void setup_views(const sgx_uniforms* u, std::uint32_t n, View<T>* out, float tol, PassCounters* counters,
+                            View<T>* host) {
     const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = make_view<T>(u[i], tol);
+    if (i < n) {
+        const View<T> v = make_view<T>(u[i], tol);
+        out[i] = v;
+        if (host != nullptr && i == 0u) *host = v;
+    }
+    if (counters != nullptr && i == 0u) *counters = PassCounters{};
 }
 
 // Final encode of a pixel's mean (geodesic_kernel.cu:502-509).
@@ -792,8 +799,9 @@ __device__ __forceinline__ float4 accum_pixel(const SmemSet<T>& m, const ViewSet
 template <class T>
 __global__ void __launch_bounds__(256) accumulate_kernel(ViewSet vs, const Rec<T>* __restrict__ results,
                                                          float4* __restrict__ acc, bool first, bool finalize,
-                                                         std::uint32_t format, void* out) {
+                                                         std::uint32_t format, void* out, CounterReport report) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (report.host != nullptr && blockIdx.x == 0u && threadIdx.x == 0u) *report.host = *report.counters;
     const SmemSet<T> m = carve<T>(smem_raw, vs.n, 0);
     load_set(m, vs, false);
     __syncthreads();
@@ -817,8 +825,9 @@ template <class T>
 __global__ void __launch_bounds__(256)
     accumulate_hdr_extract_kernel(ViewSet vs, const Rec<T>* __restrict__ results, float4* __restrict__ acc,
                                   bool first, void* out, __half2* __restrict__ ext, std::uint32_t bw,
-                                  std::uint32_t bh, float threshold) {
+                                  std::uint32_t bh, float threshold, CounterReport report) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (report.host != nullptr && blockIdx.x == 0u && threadIdx.x == 0u) *report.host = *report.counters;
     const SmemSet<T> m = carve<T>(smem_raw, vs.n, 0);
     load_set(m, vs, false);
     __syncthreads();
@@ -882,23 +891,38 @@ __global__ void encode_kernel(const float4* __restrict__ acc, std::uint32_t npix
 // ---------------------------------------------------------------------------
 // Dispatch
 // ---------------------------------------------------------------------------
+// Dynamic shared memory a kernel may use without asking.
+constexpr std::size_t kDefaultSmem = 40 * 1024;
+
 template <class T, class Ray, bool ONE>
 cudaError_t run_kernel(const PassDesc& pass, LaunchShape shape, const void* h_view, cudaStream_t st) {
     auto kern = trace_persistent<T, Ray, ONE>;
     View<T> one{};
     if constexpr (ONE) std::memcpy(&one, h_view, sizeof(View<T>));
     const std::size_t smem = set_smem_bytes<T>(pass.vs.n, pass.vs.max_S);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return e;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int threads = shape.block_threads > 0 ? shape.block_threads
                                                 : (ONE ? kDefaultBlockThreads : kDefaultBlockThreadsMulti);
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    cudaError_t e = cudaSuccess;
+    if (smem > kDefaultSmem)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    int dev = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    // the kernel's resident blocks for the last shape this thread launched
+    struct Fit {
+        int dev = -1, threads = 0, per_sm = 0, sms = 0;
+        std::size_t smem = 0;
+    };
+    static thread_local Fit fit;
+    if (fit.dev != dev || fit.threads != threads || fit.smem != smem) {
+        Fit f{dev, threads, 0, 0, smem};
+        e = cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f.per_sm, kern, threads, smem);
+        if (e != cudaSuccess) return e;
+        fit = f;
+    }
+    const int sms = fit.sms;
+    int per_sm = fit.per_sm;
     if (shape.blocks_per_sm > 0 && shape.blocks_per_sm < per_sm) per_sm = shape.blocks_per_sm;
     if (per_sm < 1) per_sm = 1;
     std::uint64_t blocks = std::uint64_t(sms) * per_sm;
@@ -1053,13 +1077,15 @@ ViewSet make_view_set(const ViewPlan& plan, const void* d_views, const std::uint
 }
 
 cudaError_t launch_setup_views(const sgx_uniforms* d_u, std::uint32_t n, void* d_views, int precision,
-                               float tol, cudaStream_t st) {
+                               float tol, cudaStream_t st, PassCounters* counters, void* host) {
     const unsigned threads = 64;
     const unsigned blocks = (n + threads - 1) / threads;
     if (precision == SGX_PRECISION_FP64) {
-        setup_views<double><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<double>*>(d_views), tol);
+        setup_views<double><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<double>*>(d_views), tol, counters,
+                                                     static_cast<View<double>*>(host));
     } else {
-        setup_views<float><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<float>*>(d_views), tol);
+        setup_views<float><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<float>*>(d_views), tol, counters,
+                                                    static_cast<View<float>*>(host));
     }
     return cudaGetLastError();
 }
@@ -1117,7 +1143,8 @@ cudaError_t launch_invariants(const void* d_view, int precision, int rhs_form, s
 }
 
 cudaError_t launch_accumulate(int precision, const ViewSet& vs, const void* results, float4* acc, bool first,
-                              bool finalize, std::uint32_t format, void* out, cudaStream_t st) {
+                              bool finalize, std::uint32_t format, void* out, cudaStream_t st,
+                              CounterReport report) {
     const unsigned threads = 256;
     const std::uint64_t blocks = (vs.total_pix + threads - 1) / threads;
     // a set of many FP64 views needs more than the default 48 KB of shared memory
@@ -1127,21 +1154,21 @@ cudaError_t launch_accumulate(int precision, const ViewSet& vs, const void* resu
                                              int(smem));
         if (e != cudaSuccess) return e;
         accumulate_kernel<double><<<unsigned(blocks), threads, smem, st>>>(
-            vs, static_cast<const Rec<double>*>(results), acc, first, finalize, format, out);
+            vs, static_cast<const Rec<double>*>(results), acc, first, finalize, format, out, report);
     } else {
         const std::size_t smem = set_smem_bytes<float>(vs.n, 0);
         cudaError_t e = cudaFuncSetAttribute(accumulate_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(smem));
         if (e != cudaSuccess) return e;
         accumulate_kernel<float><<<unsigned(blocks), threads, smem, st>>>(
-            vs, static_cast<const Rec<float>*>(results), acc, first, finalize, format, out);
+            vs, static_cast<const Rec<float>*>(results), acc, first, finalize, format, out, report);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_accumulate_hdr_extract(int precision, const ViewSet& vs, const void* results, float4* acc,
                                           bool first, void* out, void* ext, std::uint32_t W, std::uint32_t H,
-                                          float threshold, cudaStream_t st) {
+                                          float threshold, cudaStream_t st, CounterReport report) {
     if (vs.n != 1u || vs.slice_count > 1u || W < 2u || H < 2u) return cudaErrorInvalidValue;
     const std::uint32_t bw = W / 2u, bh = H / 2u;
     const std::uint64_t n = 4ull * bw * bh + (W > 2u * bw ? 2ull * bh : 0ull) + (H > 2u * bh ? W : 0u);
@@ -1151,11 +1178,11 @@ cudaError_t launch_accumulate_hdr_extract(int precision, const ViewSet& vs, cons
     if (precision == SGX_PRECISION_FP64) {
         const std::size_t smem = set_smem_bytes<double>(vs.n, 0);
         accumulate_hdr_extract_kernel<double><<<blocks, threads, smem, st>>>(
-            vs, static_cast<const Rec<double>*>(results), acc, first, out, e, bw, bh, threshold);
+            vs, static_cast<const Rec<double>*>(results), acc, first, out, e, bw, bh, threshold, report);
     } else {
         const std::size_t smem = set_smem_bytes<float>(vs.n, 0);
         accumulate_hdr_extract_kernel<float><<<blocks, threads, smem, st>>>(
-            vs, static_cast<const Rec<float>*>(results), acc, first, out, e, bw, bh, threshold);
+            vs, static_cast<const Rec<float>*>(results), acc, first, out, e, bw, bh, threshold, report);
     }
     return cudaGetLastError();
 }
