@@ -12,7 +12,7 @@
 using namespace sgxd;
 
 __device__ unsigned long long g_bad[7];
-__device__ unsigned long long g_ulp[2];
+__device__ unsigned long long g_ulp[3];
 
 __device__ __forceinline__ std::uint32_t mix(std::uint32_t x) {
     x ^= x >> 16;
@@ -135,16 +135,51 @@ __global__ void norms() {
     if (__double_as_longlong(one) != __double_as_longlong(all)) atomicAdd(&g_bad[6], 1ull);
 }
 
+// The FP64 norm against the definition evaluated with divisions, in units of
+// the last place: three products, a reciprocal and two sums, each rounded once.
+__global__ void norms64() {
+    std::uint32_t s = mix(blockIdx.x * blockDim.x + threadIdx.x + 991u);
+    auto uni = [&]() {
+        s = mix(s + 0x9e3779b9u);
+        return double(s >> 8) * 0x1p-24 + double(mix(s)) * 0x1p-56;
+    };
+    double y[6], y4[6], k4[6], k5[6];
+    const double tie = uni(), d0 = exp2(-40.0 * uni());
+    for (int i = 0; i < 6; ++i) {
+        y[i] = exp2(10.0 * uni() - 8.0) * (uni() < 0.5 ? -1.0 : 1.0);
+        y4[i] = y[i] * (1.0 + 0.01 * uni());
+        k4[i] = 2.0 * uni() - 1.0;
+        double d = exp2(-40.0 * uni());
+        if (tie < 0.3) {  // ratios equal, or nearly
+            y[i] = y[0];
+            y4[i] = y4[0];
+            d = d0 * (1.0 + 0x1p-18 * int(8.0 * uni()));
+            k4[i] = 0.0;
+        }
+        k5[i] = k4[i] - d;
+        if (tie > 0.95 && uni() < 0.3) k5[i] = k4[i];
+    }
+    auto six = [](const double* v) { return KSC<double>{v[0], v[1], v[2], v[3], v[4], v[5]}; };
+    const KAttempt<double> A{six(y4), six(k4), six(k5), exp2(-8.0 * uni())};
+    double want = 0.0;
+    for (int i = 0; i < 6; ++i)
+        want = fmax(want, fabs(A.h6 * (k4[i] - k5[i])) / (double(1e-6f) * (1.0 + fmax(fabs(y[i]), fabs(y4[i])))));
+    want = fmin(want, 1e30);
+    const long long d = __double_as_longlong(error_norm_pos(six(y), A, 1e-6f)) - __double_as_longlong(want);
+    atomicMax(&g_ulp[2], (unsigned long long)(d < 0 ? -d : d));
+}
+
 int main() {
     for (int e : {-60, -20, -3, -1, 0, 1, 2, 9, 28, 60}) single<<<(1 << 23) / 256, 256>>>(e, -30, 30);
     for (int e : {-67, -20, -1, 0, 1, 7, 16, 40}) dbl<<<(1 << 23) / 256, 256>>>(e);
     steps<<<(1 << 22) / 256, 256>>>();
     norms<<<(1 << 22) / 256, 256>>>();
-    unsigned long long bad[7], ulp[2];
+    norms64<<<(1 << 22) / 256, 256>>>();
+    unsigned long long bad[7], ulp[3];
     cudaMemcpyFromSymbol(bad, g_bad, sizeof(bad));
     cudaMemcpyFromSymbol(ulp, g_ulp, sizeof(ulp));
     if (cudaDeviceSynchronize() != cudaSuccess) return 1;
-    std::printf("%llu %llu %llu %llu %llu %llu %llu %llu %llu\n", bad[0], bad[1], bad[2], bad[3], bad[4], bad[5], bad[6], ulp[0],
-                ulp[1]);
+    std::printf("%llu %llu %llu %llu %llu %llu %llu %llu %llu %llu\n", bad[0], bad[1], bad[2], bad[3], bad[4], bad[5], bad[6], ulp[0],
+                ulp[1], ulp[2]);
     return 0;
 }

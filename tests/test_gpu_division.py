@@ -6,7 +6,8 @@ bit, for every significand of the divisor, and a fixed step that divides so
 equals one with compiled divisions, whatever the state.  The precision form's
 norm from one component is the norm over all six, bit for bit.  FP64: the Newton reciprocal is
 rounded twice (its correction and the sum), the square root likewise: within
-1 ulp of the rounded result.
+1 ulp of the rounded result.  The FP64 norm takes eight such roundings more than
+the definition's four: within 8 ulp.
 """
 
 from __future__ import annotations
@@ -27,8 +28,9 @@ def test_divisions_match_the_compilers(tmp_path, sgx):
     subprocess.run([B._nvcc(), *B.ARCH, *B.NVCC_FLAGS, str(ROOT / "tests" / "division_check.cu"), "-o", str(exe)],
                    check=True, capture_output=True, text=True)
     out = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=120).stdout
-    reciprocal, sixth, quotient, edge, kerr, schwarzschild, norm, rcp_ulp, sqrt_ulp = map(int, out.split())
+    reciprocal, sixth, quotient, edge, kerr, schwarzschild, norm, rcp_ulp, sqrt_ulp, norm_ulp = map(int, out.split())
     print(out)
     assert reciprocal == sixth == quotient == edge == 0
     assert kerr == schwarzschild == norm == 0
     assert rcp_ulp <= 1 and sqrt_ulp <= 1
+    assert norm_ulp <= 8
