@@ -44,6 +44,10 @@ constexpr int kCkDense = 10;
 // 32.1 / 33.3; FP32 crossing model 8,192 rays 0.96 / 0.62, 49,152 1.2 / 1.1.
 constexpr int kThreads = 128, kSmallThreads = 32;
 constexpr std::uint64_t kSmallForward = 1u << 18, kSmallBackward = 1u << 16;  // fewer rays: one-warp blocks
+// Warps an SM has to hold in the backward kernels (their comment says why).
+template <class T, bool SLAB, bool DUALJ, int CK>
+constexpr int kBackwardWarps = sizeof(T) == 8 || DUALJ ? 8 : CK == kCkSparse && !SLAB ? 16 : 12;
+constexpr std::uint64_t kOneWaveBackward = 8 * 32 * 152;  // rays that 8 warps an SM hold at once
 constexpr int kMaxCross = 8;  // crossings recorded per ray (crossing model)
 constexpr int NS = 8;         // state: r, theta, phi, p_r, p_theta, psi (swept angle), sin(theta), cos(theta)
 constexpr int NC = NS + 1;    // checkpoint: state and transmittance
@@ -829,8 +833,21 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // thread laid out [slot][value][thread] (consecutive threads, consecutive
 // words); CK = kCkSparse in a thread-local array.  Launched with at most TH
 // threads a block, exactly TH where the segment is shared.
-template <class T, bool SLAB, bool DUALJ, int CK, int TH>
-__global__ void __launch_bounds__(TH, (sizeof(T) == 8 ? 256 : 512) / TH)
+//
+// W is the number of warps that an SM has to hold, which caps the registers at
+// 65,536 / (32 W).  The FP32 sweep issues well with few warps and its arithmetic
+// has independent chains, so registers for more of them in flight are worth more
+// than warps.  Backward call on one GB300, ms, at W = 16 (128 registers) / W as
+// chosen: slab 512 x 512 x 4 spp 6.38 / 6.05, crossings 512 x 512 x 4 1.70 / 1.59
+// (W = 12; 14, 10 and 8 within 1 %); one-warp blocks 160 x 96 x 4 0.80 / 0.59,
+// 255 x 193 crossings 0.57 / 0.50 (W = 10).  Up to 38,912 rays 8 warps an SM hold
+// them all at once, and 224 registers take 64 x 64 x 4 from 0.34 (W = 10) to
+// 0.32; above that line they need a second wave (160 x 96 x 4: 0.71).  In the
+// sparse form W = 12 takes the slab from 6.61 to 6.48, but the crossings, whose
+// segment is their main traffic, from 1.63 to 1.65: they stay at 16.  The dual
+// numbers spill 3 KB a thread at 128 registers and 0.9 KB at 255: 80 / 47.
+template <class T, bool SLAB, bool DUALJ, int CK, int TH, int W = kBackwardWarps<T, SLAB, DUALJ, CK>>
+__global__ void __launch_bounds__(TH, W * 32 / TH)
     diff_backward_kernel(DiffConst<T> k, DiffParamsT<T> p, DiffBufs<T> b, const float* __restrict__ gimg) {
     constexpr bool SHARED = CK == kCkDense;
     extern __shared__ __align__(16) unsigned char diff_seg_raw[];
@@ -1274,8 +1291,11 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
             const int smem = (kCkDense + 1) * NC * th * int(sizeof(T));
             auto* kern = th == kThreads ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kThreads>
                                                 : diff_backward_kernel<T, false, false, kCkDense, kThreads>)
-                                        : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads>
-                                                : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads>);
+                         : st.n > kOneWaveBackward
+                             ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 10>
+                                     : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, 10>)
+                             : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 8>
+                                     : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, 8>);
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             kern<<<grid, th, smem, s>>>(k, p, b, gimg);
