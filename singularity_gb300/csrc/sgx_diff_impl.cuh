@@ -41,12 +41,16 @@ constexpr int kCkDense = 10;
 // GB300): forward FP32 65,536 rays 0.53 / 0.46, 131,072 rays 0.72 / 0.66,
 // 262,144 1.05 / 1.04, 524,288 1.73 / 1.73; FP64 65,536 rays 18.2 / 13.9, 131,072
 // 27.4 / 27.5; backward FP64 8,192 rays 13.1 / 12.4, 32,768 21.1 / 18.6, 65,536
-// 32.1 / 33.3; FP32 crossing model 8,192 rays 0.96 / 0.62, 49,152 1.2 / 1.1.
+// 32.1 / 33.3; FP32 64-step checkpoints 262,144 rays 1.97 / 2.01, 1,048,576
+// crossings 5.27 / 5.31.  The FP32 backward over 10-step checkpoints runs one-warp
+// blocks at every size, since the next block need not wait for the slowest of
+// four warps: slab 65,536 rays 0.75 / 0.58, 1,048,576 6.06 / 5.75, 2,097,152 14.1 /
+// 13.4, crossings 1,048,576 5.01 / 4.84.
 constexpr int kThreads = 128, kSmallThreads = 32;
 constexpr std::uint64_t kSmallForward = 1u << 18, kSmallBackward = 1u << 16;  // fewer rays: one-warp blocks
 // Warps an SM has to hold in the backward kernels (their comment says why).
 template <class T, bool SLAB, bool DUALJ, int CK>
-constexpr int kBackwardWarps = sizeof(T) == 8 || DUALJ ? 8 : CK == kCkSparse && !SLAB ? 16 : 12;
+constexpr int kBackwardWarps = sizeof(T) == 8 || DUALJ ? 8 : CK == kCkDense ? 10 : SLAB ? 12 : 16;
 constexpr std::uint64_t kOneWaveBackward = 8 * 32 * 152;  // rays that 8 warps an SM hold at once
 constexpr int kMaxCross = 8;  // crossings recorded per ray (crossing model)
 constexpr int NS = 8;         // state: r, theta, phi, p_r, p_theta, psi (swept angle), sin(theta), cos(theta)
@@ -835,17 +839,16 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // threads a block, exactly TH where the segment is shared.
 //
 // W is the number of warps that an SM has to hold, which caps the registers at
-// 65,536 / (32 W).  The FP32 sweep issues well with few warps and its arithmetic
-// has independent chains, so registers for more of them in flight are worth more
-// than warps.  Backward call on one GB300, ms, at W = 16 (128 registers) / W as
-// chosen: slab 512 x 512 x 4 spp 6.38 / 6.05, crossings 512 x 512 x 4 1.70 / 1.59
-// (W = 12; 14, 10 and 8 within 1 %); one-warp blocks 160 x 96 x 4 0.80 / 0.59,
-// 255 x 193 crossings 0.57 / 0.50 (W = 10).  Up to 38,912 rays 8 warps an SM hold
-// them all at once, and 224 registers take 64 x 64 x 4 from 0.34 (W = 10) to
-// 0.32; above that line they need a second wave (160 x 96 x 4: 0.71).  In the
-// sparse form W = 12 takes the slab from 6.61 to 6.48, but the crossings, whose
-// segment is their main traffic, from 1.63 to 1.65: they stay at 16.  The dual
-// numbers spill 3 KB a thread at 128 registers and 0.9 KB at 255: 80 / 47.
+// 65,536 / (32 W).  The FP32 sweep's arithmetic has independent chains, so
+// registers for more of them in flight are worth more than warps.  Backward call
+// on one GB300, ms, at W = 16 (128 registers) / W = 10 (168, 12 warps resident):
+// one-warp blocks 160 x 96 x 4 spp 0.80 / 0.59, 255 x 193 crossings 0.57 / 0.50;
+// 128-thread blocks 512 x 512 x 4 6.38 / 6.05.  Up to 38,912 rays 8 warps an SM
+// hold them all at once, and 224 registers take 64 x 64 x 4 from 0.34 to 0.32;
+// above that line they need a second wave (160 x 96 x 4: 0.71).  In the sparse
+// form W = 12 takes the slab from 6.61 to 6.48, but the crossings, whose segment
+// is their main traffic, from 1.63 to 1.65: they stay at 16.  The dual numbers
+// spill 3 KB a thread at 128 registers and 0.9 KB at 255: 80 / 47.
 template <class T, bool SLAB, bool DUALJ, int CK, int TH, int W = kBackwardWarps<T, SLAB, DUALJ, CK>>
 __global__ void __launch_bounds__(TH, W * 32 / TH)
     diff_backward_kernel(DiffConst<T> k, DiffParamsT<T> p, DiffBufs<T> b, const float* __restrict__ gimg) {
@@ -1280,20 +1283,18 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
     const DiffParamsT<T> p{T(st.p.spin), T(st.p.incl), T(st.p.r_in), T(st.p.t_scale)};
     DiffBufs<T> b = carve_bufs<T>(st, k.spp);
     const bool slab = st.o.model == SGX_DIFF_MODEL_SLAB, dual = st.o.adjoint_form == SGX_DIFF_ADJOINT_DUAL;
-    const int th = st.n < kSmallBackward ? kSmallThreads : kThreads;
-    const unsigned grid = unsigned((st.n + th - 1) / th);
     bool dense = false;
+    if constexpr (sizeof(T) == 4) dense = st.ck == std::uint32_t(kCkDense);
+    const int th = dense || st.n < kSmallBackward ? kSmallThreads : kThreads;
+    const unsigned grid = unsigned((st.n + th - 1) / th);
     if constexpr (sizeof(T) == 4) {
         // the dense checkpoints pair with the hand-derived reverse pass only;
         // their segments are laid out for the block size
-        dense = st.ck == std::uint32_t(kCkDense);
         if (dense) {
             const int smem = (kCkDense + 1) * NC * th * int(sizeof(T));
-            auto* kern = th == kThreads ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kThreads>
-                                                : diff_backward_kernel<T, false, false, kCkDense, kThreads>)
-                         : st.n > kOneWaveBackward
-                             ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 10>
-                                     : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, 10>)
+            auto* kern = st.n > kOneWaveBackward
+                             ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads>
+                                     : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads>)
                              : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 8>
                                      : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, 8>);
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -1,7 +1,7 @@
 """The FP32 backward kernels at the edges of the launch rule.
 
 The sizes are the last rays of a rule and the first of the next: 8 warps on
-each of 152 SMs, and the change from one-warp to four-warp blocks.  The dense
+each of 152 SMs, and the sparse form's change from one-warp to four-warp blocks.  The dense
 and the sparse checkpoints replay the same steps in different kernels, so the
 gradients differ by FP32 rounding alone: about 300 steps of 6e-8 each, 2e-5 of
 the largest component.
