@@ -393,7 +393,9 @@ void sgx_diff_opts_default(sgx_diff_opts* opts);
  * from `base` (a Kerr uniform block), into d_image (device, W*H*3 floats; NULL:
  * an internal buffer) and keeps what the backward pass needs (a state and
  * transmittance checkpoint every C = opts->checkpoint_interval steps,
- * (max_steps/C + 1) * 9 values per ray).  Synchronous. */
+ * (max_steps/C + 1) * 9 values per ray; for the crossing model also 8 * 5
+ * values, and 8 * 7 more for the reverse pass where they fit the 16 GiB too,
+ * which the backward pass otherwise forms again).  Synchronous. */
 sgx_status sgx_diff_forward(sgx_context* ctx, const sgx_uniforms* base, const sgx_diff_params* params,
                             const sgx_diff_opts* opts, float* d_image, void* stream);
 /* Backward pass of the last forward: d_grad_image (device, W*H*3 floats) is

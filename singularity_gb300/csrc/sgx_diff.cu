@@ -116,15 +116,28 @@ sgx_status sgx_diff_forward(sgx_context* c, const sgx_uniforms* base, const sgx_
     if (need > limit)
         return fail(c, SGX_ERR_INVALID_ARGUMENT, "differentiable render needs " + std::to_string(need >> 20) +
                                                      " MiB of records: fewer rays or max_steps");
-    const std::size_t all = need + (o.precision == SGX_PRECISION_FP64 ? crossing_bytes<double>(st.n, st.nx)
-                                                                      : crossing_bytes<float>(st.n, st.nx));
+    // The crossing states that the reverse pass forms its seeds from lie behind
+    // the records where the limit (and the device) has room for both; without
+    // them the sweep forms the seeds from the states it rebuilds, and what is
+    // accepted depends on the records alone.
+    const std::size_t extra = o.precision == SGX_PRECISION_FP64 ? crossing_bytes<double>(st.n, st.nx)
+                                                                : crossing_bytes<float>(st.n, st.nx);
+    st.xs = o.model == SGX_DIFF_MODEL_CROSSING && o.adjoint_form == SGX_DIFF_ADJOINT_REVERSE && need + extra <= limit;
+    const std::size_t all = need + (st.xs ? extra : 0);
     if (st.cap < all) {
         if (st.mem) cudaFree(st.mem);
         st.mem = nullptr;
         st.cap = 0;
-        cudaError_t e = cudaMalloc(&st.mem, all);
+        std::size_t got = all;
+        cudaError_t e = cudaMalloc(&st.mem, got);
+        if (e == cudaErrorMemoryAllocation && st.xs) {
+            (void)cudaGetLastError();
+            st.xs = false;
+            got = need;
+            e = cudaMalloc(&st.mem, got);
+        }
         if (e != cudaSuccess) return cuda_fail(c, e, "sgx_diff_forward: cudaMalloc");
-        st.cap = all;
+        st.cap = got;
     }
     const std::size_t img_bytes = std::size_t(base->width) * base->height * 3 * sizeof(float);
     if (d_image == nullptr) {

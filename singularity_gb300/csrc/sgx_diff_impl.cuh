@@ -79,6 +79,7 @@ template <class T> struct DiffBufs {
     T* xw;              // [kMaxCross][n]
     T* xc;              // [kMaxCross][3][n]
     T* xs;              // [kMaxCross][7][n]: r, theta, psi before and r, theta, phi, psi after the crossing step
+                        // (nullptr: not kept, the sweep forms a crossing's seeds from the states it rebuilds)
     double* grads;      // [4][n]
     const T* ox;        // [spp] sub-pixel offsets
     const T* oy;
@@ -726,9 +727,11 @@ __global__ void __launch_bounds__(128) diff_forward_kernel(DiffConst<T> k, DiffP
                                 b.xw[std::uint64_t(nc) * b.n + id] = w;
 #pragma unroll
                                 for (int c = 0; c < 3; ++c) b.xc[(std::uint64_t(nc) * 3 + c) * b.n + id] = col[c];
-                                const T xs[7] = {prev[0], prev[1], prev[5], y[0], y[1], y[2], y[5]};
+                                if (b.xs != nullptr) {
+                                    const T xs[7] = {prev[0], prev[1], prev[5], y[0], y[1], y[2], y[5]};
 #pragma unroll
-                                for (int c = 0; c < 7; ++c) b.xs[(std::uint64_t(nc) * 7 + c) * b.n + id] = xs[c];
+                                    for (int c = 0; c < 7; ++c) b.xs[(std::uint64_t(nc) * 7 + c) * b.n + id] = xs[c];
+                                }
                             } else {
                                 atomicAdd(b.overflow, 1ull);
                             }
@@ -849,7 +852,11 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // form W = 12 takes the slab from 6.61 to 6.48, but the crossings, whose segment
 // is their main traffic, from 1.63 to 1.65: they stay at 16.  The dual numbers
 // spill 3 KB a thread at 128 registers and 0.9 KB at 255: 80 / 47.
-template <class T, bool SLAB, bool DUALJ, int CK, int TH, int W = kBackwardWarps<T, SLAB, DUALJ, CK>>
+//
+// XS: the forward stored the crossing states.  Without them (records at the
+// memory limit) the crossing model's seeds are formed in the sweep.
+template <class T, bool SLAB, bool DUALJ, int CK, int TH, int W = kBackwardWarps<T, SLAB, DUALJ, CK>,
+          bool XS = !SLAB && !DUALJ>
 __global__ void __launch_bounds__(TH, W * 32 / TH)
     diff_backward_kernel(DiffConst<T> k, DiffParamsT<T> p, DiffBufs<T> b, const float* __restrict__ gimg) {
     constexpr bool SHARED = CK == kCkDense;
@@ -899,7 +906,7 @@ __global__ void __launch_bounds__(TH, W * 32 / TH)
     // colour one after another.
     T xcs[kMaxCross], xgw[kMaxCross];
     std::uint32_t xkk[kMaxCross];
-    [[maybe_unused]] T xq[!SLAB && !DUALJ ? kMaxCross : 1][7];
+    [[maybe_unused]] T xq[XS ? kMaxCross : 1][7];
     if constexpr (!SLAB) {
         T w[kMaxCross], c3[kMaxCross][3], tau_j[kMaxCross];
         T tau = T(1);
@@ -918,7 +925,7 @@ __global__ void __launch_bounds__(TH, W * 32 / TH)
 #pragma unroll
             for (int c = 0; c < 3; ++c) R[c] = w[j] * c3[j][c] + (T(1) - w[j]) * R[c];
         }
-        if constexpr (!DUALJ) {
+        if constexpr (XS) {
             for (std::uint32_t j = 0; j < nc; ++j) {
                 T x[7], q[11];
 #pragma unroll
@@ -1057,7 +1064,20 @@ __global__ void __launch_bounds__(TH, W * 32 / TH)
                 }
             } else if constexpr (!DUALJ) {
                 if (jx >= 0 && kk == xkk[jx]) {
-                    const T* q = xq[jx--];
+                    const T* q;
+                    [[maybe_unused]] T qv[11];
+                    if constexpr (XS) {
+                        q = xq[jx];
+                    } else {
+                        crossing_vjp<T>(yp[0], yp[1], yp[5], yc[0], yc[1], yc[2], yc[5], L, a, r_in, p.t_scale, k, g,
+                                        xcs[jx], xgw[jx], qv);
+                        q = qv;
+                        muL += qv[7];
+                        g_a += qv[8] * k.M;
+                        g_rin += qv[9] * k.M;
+                        g_ts += qv[10];
+                    }
+                    --jx;
                     pend[0] += q[0];
                     pend[1] += q[1];
                     pend[5] += q[2];
@@ -1197,6 +1217,7 @@ struct sgx_diff_state {
     std::uint32_t ck = kCkSparse;  // steps between checkpoints (kCkSparse or kCkDense)
     std::uint32_t precision = SGX_PRECISION_FP32;
     std::uint32_t nx = kMaxCross;  // crossing records per ray (1 for the slab model)
+    bool xs = false;               // crossing states kept behind the records
     sgx_uniforms u{};
     sgx_diff_params p{};
     sgx_diff_opts o{};
@@ -1217,11 +1238,8 @@ std::size_t state_bytes(std::uint64_t n, std::uint32_t slots, std::uint32_t spp,
            r(4 * ((n + 1023) / 1024) * 8) + 256;
 }
 
-// Bytes of the crossing states (after state_bytes; not counted against the
-// form's memory budget, which decides what is accepted and at which interval).
-template <class T> std::size_t crossing_bytes(std::uint64_t n, std::size_t nx) {
-    return nx > 1 ? nx * 7 * n * sizeof(T) : 0;
-}
+// Bytes of the crossing states (after state_bytes).
+template <class T> std::size_t crossing_bytes(std::uint64_t n, std::size_t nx) { return nx * 7 * n * sizeof(T); }
 
 template <class T>
 DiffBufs<T> carve_bufs(sgx_diff_state& st, std::uint32_t spp) {
@@ -1248,8 +1266,8 @@ DiffBufs<T> carve_bufs(sgx_diff_state& st, std::uint32_t spp) {
     b.ox = off;
     b.oy = off + spp;
     b.overflow = reinterpret_cast<unsigned long long*>(take(64));
-    b.xs = nx > 1 ? reinterpret_cast<T*>(static_cast<unsigned char*>(st.mem) + state_bytes<T>(n, st.slots, spp, nx))
-                  : nullptr;
+    b.xs = st.xs ? reinterpret_cast<T*>(static_cast<unsigned char*>(st.mem) + state_bytes<T>(n, st.slots, spp, nx))
+                 : nullptr;
     return b;
 }
 
@@ -1292,7 +1310,9 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
         // their segments are laid out for the block size
         if (dense) {
             const int smem = (kCkDense + 1) * NC * th * int(sizeof(T));
-            auto* kern = st.n > kOneWaveBackward
+            constexpr int kW = kBackwardWarps<T, false, false, kCkDense>;
+            auto* kern = !slab && !st.xs ? diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, kW, false>
+                         : st.n > kOneWaveBackward
                              ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads>
                                      : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads>)
                              : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 8>
@@ -1305,7 +1325,10 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
     if (!dense) {
         if (slab && !dual) diff_backward_kernel<T, true, false, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
         else if (slab) diff_backward_kernel<T, true, true, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
-        else if (!dual) diff_backward_kernel<T, false, false, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
+        else if (!dual && st.xs) diff_backward_kernel<T, false, false, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
+        else if (!dual)
+            diff_backward_kernel<T, false, false, kCkSparse, kThreads, kBackwardWarps<T, false, false, kCkSparse>, false>
+                <<<grid, th, 0, s>>>(k, p, b, gimg);
         else diff_backward_kernel<T, false, true, kCkSparse, kThreads><<<grid, th, 0, s>>>(k, p, b, gimg);
     }
     const std::uint32_t nchunks = std::uint32_t((st.n + 1023) / 1024);
