@@ -76,7 +76,7 @@ __host__ __device__ inline std::uint32_t slice_row(std::uint32_t band, std::uint
 constexpr std::uint32_t kDefaultRefill = 128;
 constexpr int kDefaultBlockThreads = 64;
 // Multi-view passes copy the whole view table into each block's shared memory
-// (64 views: 18 KB), so small blocks run out of shared memory before
+// (64 views: 16 KB), so small blocks run out of shared memory before
 // registers: 64 batched views at 64-thread blocks fit 24 warps per SM, at 128
 // threads 28 (register-limited); 1866 against 2003 Mrays/s.
 constexpr int kDefaultBlockThreadsMulti = 128;

@@ -102,7 +102,7 @@ template <class T, int FL> struct KerrFixed {
     std::uint32_t steps, term;
     static constexpr std::uint32_t rej = 0, zone = 0;
 
-    __device__ __forceinline__ bool init(const View<T>& v, const CamDir<T>& cd, const PassDesc&) {
+    __device__ __forceinline__ bool init(const View<T>& v, const CamFP64<T>& d, const CamDir<T>& cd, const PassDesc&) {
         steps = 0;
         T E, L;
         if (!kerr_init(v, cd, y, E, L)) {
@@ -177,7 +177,7 @@ template <class T, int FL> struct SchwFixed {
     std::uint32_t steps, term;
     static constexpr std::uint32_t rej = 0, zone = 0;
 
-    __device__ __forceinline__ bool init(const View<T>& v, const CamDir<T>& cd, const PassDesc&) {
+    __device__ __forceinline__ bool init(const View<T>& v, const CamFP64<T>& d, const CamDir<T>& cd, const PassDesc&) {
         steps = 0;
         y = schw_init(v, cd);
         prev_th = y.th;
@@ -259,7 +259,7 @@ template <class T, int FL> struct KerrAdaptive {
     T t0, t1, t2;
     std::uint32_t steps, term, rej, zone;
 
-    __device__ __forceinline__ bool init(const View<T>& v, const CamDir<T>& cd, const PassDesc& pass) {
+    __device__ __forceinline__ bool init(const View<T>& v, const CamFP64<T>& d, const CamDir<T>& cd, const PassDesc& pass) {
         steps = rej = zone = 0;
         T E, L;
         KS<T> y0;
@@ -270,7 +270,7 @@ template <class T, int FL> struct KerrAdaptive {
         y = KSC<T>{y0.r, v.sin_th, v.cos_th, y0.ph, y0.pr, y0.pth};
         if constexpr (MIXED) {
             double Ed, Ld, prd, pthd;
-            if (!kerr_init_fp64_constants(v, cd, Ed, Ld, prd, pthd)) {
+            if (!kerr_init_fp64_constants(d, cd, Ed, Ld, prd, pthd)) {
                 term = TERM_NO_ROOT;
                 return false;
             }
@@ -278,7 +278,7 @@ template <class T, int FL> struct KerrAdaptive {
             L = float(Ld);
             y.pr = float(prd);
             y.pth = float(pthd);
-            Q = float(carter_Q_fp64(v, Ed, Ld, pthd));
+            Q = float(carter_Q_fp64(d, Ed, Ld, pthd));
         } else {
             Q = carter_Q(v, E, L, y.pth);
         }
@@ -549,7 +549,7 @@ enum : int { MODE_IDLE = 0, MODE_ACTIVE = 1, MODE_DONE = 2 };
 // shared-memory loads held in registers.
 template <class T, class Ray, bool ONE>
 __global__ void __maxnreg__(ONE ? Ray::kRegs : Ray::kRegsMulti)
-    trace_persistent(const __grid_constant__ PassDesc pass, const __grid_constant__ View<T> one) {
+    trace_persistent(const __grid_constant__ PassDesc pass, const __grid_constant__ ViewSlot<T> one) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // Block totals of the ray counters and each lane's record slot live in
     // shared memory, not in registers held across the integration loop.
@@ -569,7 +569,7 @@ __global__ void __maxnreg__(ONE ? Ray::kRegs : Ray::kRegsMulti)
     std::uint32_t vid = 0;
     bool exhausted = false;
     auto view_of = [&](std::uint32_t i) -> const View<T>& {
-        if constexpr (ONE) return one;
+        if constexpr (ONE) return one.v;
         else return m.views[i];
     };
 
@@ -598,6 +598,7 @@ __global__ void __maxnreg__(ONE ? Ray::kRegs : Ray::kRegsMulti)
                     if (id < vs.total_rays) {
                         vid = (ONE || vs.n == 1u) ? 0u : find_view(m.ray_off, vs.n, id);
                         const View<T>& v = view_of(vid);
+                        const CamFP64<T>& cam = ONE ? one.d : cam_of<T>(vs.views, vs.n)[vid];
                         const std::uint32_t Sv = m.S[vid];
                         const std::uint64_t local = id - m.ray_off[vid];
                         const std::uint64_t seq = local / Sv;
@@ -624,7 +625,7 @@ __global__ void __maxnreg__(ONE ? Ray::kRegs : Ray::kRegsMulti)
                             const T ox = v.spp == 1u ? DLIT(0.5) : m.off_x[sl];
                             const T oy = v.spp == 1u ? DLIT(0.5) : m.off_y[sl];
                             const CamDir<T> cd = camera_dir(v, gx, gy, ox, oy);
-                            mode = ray.init(v, cd, pass) ? MODE_ACTIVE : MODE_DONE;
+                            mode = ray.init(v, cam, cd, pass) ? MODE_ACTIVE : MODE_DONE;
                         }
                     }
                 }
@@ -667,7 +668,8 @@ __global__ void __launch_bounds__(128) trace_probe(const View<T>* __restrict__ g
     T ox, oy;
     sample_offset<T>(v.spp, s[i], ox, oy);
     const CamDir<T> cd = camera_dir(v, gx[i], gy[i], ox, oy);
-    if (ray.init(v, cd, pass)) run_ray<T>(ray, v, pass, v.max_steps);
+    const CamFP64<T>& d = *cam_of<T>(g_view, 1);
+    if (ray.init(v, d, cd, pass)) run_ray<T>(ray, v, pass, v.max_steps);
     const V3<T> hdr = shade_record(v, ray.record());
     if (hdr3 != nullptr) {
         hdr3[3 * i + 0] = float(hdr.x);
@@ -698,7 +700,8 @@ __global__ void __launch_bounds__(128) trace_invariants(const View<T>* __restric
     sample_offset<T>(v.spp, s[i], ox, oy);
     const CamDir<T> cd = camera_dir(v, gx[i], gy[i], ox, oy);
     Ray ray;
-    if (ray.init(v, cd, pass)) run_ray<T>(ray, v, pass, v.max_steps);
+    const CamFP64<T>& d = *cam_of<T>(g_view, 1);
+    if (ray.init(v, d, cd, pass)) run_ray<T>(ray, v, pass, v.max_steps);
     double* o = inv5 + 5 * i;
     if (ray.term == TERM_NO_ROOT) {
         for (int k = 0; k < 5; ++k) o[k] = __longlong_as_double(0x7ff8000000000000ll);  // NaN
@@ -709,8 +712,8 @@ __global__ void __launch_bounds__(128) trace_invariants(const View<T>* __restric
         double E, L, Q0;
         if constexpr (Ray::MIXED) {
             double prd, pthd;
-            kerr_init_fp64_constants(v, cd, E, L, prd, pthd);
-            Q0 = carter_Q_fp64(v, E, L, pthd);
+            kerr_init_fp64_constants(d, cd, E, L, prd, pthd);
+            Q0 = carter_Q_fp64(d, E, L, pthd);
         } else {
             E = double(Ef);
             L = double(Lf);
@@ -730,12 +733,15 @@ __global__ void __launch_bounds__(128) trace_invariants(const View<T>* __restric
 
 template <class T>
 __global__ void setup_views(const sgx_uniforms* u, std::uint32_t n, View<T>* out, float tol, PassCounters* counters,
-                            View<T>* host) {
+                            ViewSlot<T>* host) {
     const std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const View<T> v = make_view<T>(u[i], tol);
+        const CamFP64<T> d = make_cam(v);
         out[i] = v;
-        if (host != nullptr && i == 0u) *host = v;
+        if constexpr (!std::is_empty_v<CamFP64<T>>)
+            reinterpret_cast<CamFP64<T>*>(reinterpret_cast<unsigned char*>(out) + cam_offset<T>(n))[i] = d;
+        if (host != nullptr && i == 0u) *host = ViewSlot<T>{v, d};
     }
     if (counters != nullptr && i == 0u) *counters = PassCounters{};
 }
@@ -897,8 +903,8 @@ constexpr std::size_t kDefaultSmem = 40 * 1024;
 template <class T, class Ray, bool ONE>
 cudaError_t run_kernel(const PassDesc& pass, LaunchShape shape, const void* h_view, cudaStream_t st) {
     auto kern = trace_persistent<T, Ray, ONE>;
-    View<T> one{};
-    if constexpr (ONE) std::memcpy(&one, h_view, sizeof(View<T>));
+    ViewSlot<T> one{};
+    if constexpr (ONE) std::memcpy(&one, h_view, sizeof(one));
     const std::size_t smem = set_smem_bytes<T>(pass.vs.n, pass.vs.max_S);
     const int threads = shape.block_threads > 0 ? shape.block_threads
                                                 : (ONE ? kDefaultBlockThreads : kDefaultBlockThreadsMulti);
@@ -993,8 +999,9 @@ cudaError_t dispatch(int metric, int precision, int integrator, int rhs_form, F&
 
 }  // namespace
 
+// Room for one view; n of them hold a set of n (cam_offset).
 std::size_t view_bytes() {
-    const std::size_t a = sizeof(View<float>), b = sizeof(View<double>);
+    const std::size_t a = sizeof(ViewSlot<float>), b = sizeof(ViewSlot<double>);
     return ((a > b ? a : b) + 255) / 256 * 256;
 }
 
@@ -1082,10 +1089,10 @@ cudaError_t launch_setup_views(const sgx_uniforms* d_u, std::uint32_t n, void* d
     const unsigned blocks = (n + threads - 1) / threads;
     if (precision == SGX_PRECISION_FP64) {
         setup_views<double><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<double>*>(d_views), tol, counters,
-                                                     static_cast<View<double>*>(host));
+                                                     static_cast<ViewSlot<double>*>(host));
     } else {
         setup_views<float><<<blocks, threads, 0, st>>>(d_u, n, static_cast<View<float>*>(d_views), tol, counters,
-                                                    static_cast<View<float>*>(host));
+                                                    static_cast<ViewSlot<float>*>(host));
     }
     return cudaGetLastError();
 }
