@@ -251,7 +251,7 @@ sgx_status render_impl(sgx_context* c, const sgx_uniforms* u, const sgx_render_o
         pass.zone = o.fp64_zone;
         pass.project = o.projection;
         SGX_CUDA(c, cudaEventRecord(c->ev_trace0, st));
-        sgxk::LaunchShape shape{int(o.block_threads), int(o.blocks_per_sm)};
+        sgxk::LaunchShape shape{int(o.block_threads), int(o.blocks_per_sm), sgxk::shared_div(*u)};
         SGX_CUDA(c, sgxk::launch_trace(int(u->metric_type), int(o.precision), int(o.integrator), int(o.rhs_form),
                                        pass, shape, st, c->h_view));
         SGX_CUDA(c, cudaEventRecord(c->ev_trace1, st));

@@ -96,6 +96,9 @@ struct PassDesc {
 struct LaunchShape {
     int block_threads;
     int blocks_per_sm;
+    // FP32 Kerr steps with the reference's divisions: whether a single view takes
+    // them from shared reciprocals (shared_div_holds)
+    bool shared_div = true;
 };
 
 // Counters of a finished pass and the pinned host copy an accumulation makes of
@@ -104,6 +107,9 @@ struct CounterReport {
     const PassCounters* counters = nullptr;
     PassCounters* host = nullptr;
 };
+
+// shared_div_holds of a view (LaunchShape::shared_div).
+bool shared_div(const sgx_uniforms& u);
 
 // Host plan of a ViewSet: the layout block's contents (to copy to the device
 // as one array of 64-bit words) and the totals.  S_pass == 0 -> every view's

@@ -87,8 +87,9 @@ constexpr int FL_DIV = 32;
 // Kerr, fixed step (geodesic_kernel.cu:303-403).
 template <class T, int FL> struct KerrFixed {
     // 56 registers (36 warps an SM): 1080p x 16 44.8 -> 44.3 ms, the reference
-    // form 1279 x 719 x 4 12.9 -> 12.6 ms; 48 spill (47.1, 14.5 ms)
-    static constexpr int kRegs = sizeof(T) == 4 ? ((FL & FL_SC) ? 64 : 56) : 255;
+    // form 1279 x 719 x 4 12.9 -> 12.6 ms; 48 spill (47.1, 14.5 ms).  With the plain
+    // divisions 64 (1279 x 719 x 2 11.7 ms, 12.2 at 56)
+    static constexpr int kRegs = sizeof(T) == 4 ? ((FL & FL_SC) || FL == 0 ? 64 : 56) : 255;
     static constexpr int kRegsMulti = sizeof(T) == 4 ? 64 : 255;
     static constexpr bool kCountDown = false;
     static constexpr bool FAST = (FL & FL_FAST) != 0;
@@ -944,6 +945,13 @@ cudaError_t run_persistent(const PassDesc& pass, LaunchShape shape, const void* 
     constexpr bool kDivides = std::is_same_v<T, float> && !kAdaptive &&
                               (FL == 0 || std::is_same_v<Policy<T, FL>, SchwFixed<T, FL>>);
     constexpr int FL1 = kDivides ? (FL | FL_DIV) : FL;
+    if constexpr (kDivides && std::is_same_v<Policy<T, FL>, KerrFixed<T, FL>>) {
+        // a Kerr view out of the shared reciprocals' range: the plain expressions
+        // (M = 400 13.3 ms, 14.1 by the way out of kerr_step_ref; Schwarzschild,
+        // whose way out is the faster one, M = 1400 5.8 against 6.2)
+        if (!shape.shared_div && h_view != nullptr && pass.vs.n == 1u)
+            return run_kernel<T, Policy<T, FL>, true>(pass, shape, h_view, st);
+    }
     if (h_view != nullptr && pass.vs.n == 1u) return run_kernel<T, Policy<T, FL1>, true>(pass, shape, h_view, st);
     // the multi-view kernels of the error-controlled form take the range test
     constexpr int FLM = kAdaptive ? (FL | FL_RANGE) : FL1;
@@ -1012,6 +1020,8 @@ std::size_t record_bytes(int precision) {
 std::size_t format_bytes(std::uint32_t format) {
     return format == SGX_FORMAT_RGBA8_SRGB ? 4 : (format == SGX_FORMAT_RGBA16F_HDR ? 8 : 16);
 }
+
+bool shared_div(const sgx_uniforms& u) { return shared_div_holds(u); }
 
 bool plan_views(const sgx_uniforms* u, std::uint32_t n, std::uint32_t s0, std::uint32_t S_pass, std::uint32_t tile_w,
                 std::uint32_t tile_h, ViewPlan& plan, SliceSpec slice) {
