@@ -1,12 +1,14 @@
 // Test program (built and run by tests/test_gpu_rounding.py): tests/division_check.cu
-// with its launches and copies checked, x / 6 in FP64 and at the ends of
-// the exponent range, and the exact errors of the FP64 reciprocal and root.  Every kernel counts what it compared.  Prints division_check's line, then mismatches,
+// with its launches and copies checked, and the same arithmetic where it is
+// hardest or leaves the ordinary: quotients nearest to a rounding boundary,
+// the ends of the exponent range, x / 6 in FP64, momenta and angular momenta down
+// to the subnormals.  Every kernel counts what it compared.  Prints division_check's line, then mismatches,
 // comparisons and worst errors (in thousandths of a unit in the last place).
 #define main division_main
 #include "division_check.cu"
 #undef main
 
-enum { SIXTH_F, SIXTH_D, N_CHECKS };
+enum { HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW, N_CHECKS };
 __device__ unsigned long long g_miss[N_CHECKS], g_done[N_CHECKS], g_milli[2];
 
 __device__ __forceinline__ void count(int k, bool ok) {
@@ -16,6 +18,37 @@ __device__ __forceinline__ void count(int k, bool ok) {
 __device__ __forceinline__ bool bits_equal(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
 __device__ __forceinline__ bool bits_equal(double a, double b) {
     return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
+// For every divisor significand B the numerators A with A 2^k = B M + r, M odd of
+// 25 bits and |r| <= 7: quotients r / (B M) from the midpoint of two floats.
+// B = 2^t B', B' odd, leaves r = 2^t r', so t <= 2, and 2^t solutions M of
+// M = -r' / B' mod 2^(k - t).  Exponents ea, eb of numerator and divisor.
+__global__ void hard(int ea, int eb) {
+    const std::uint32_t B = 0x800000u + blockIdx.x * blockDim.x + threadIdx.x;  // 2^23 of them
+    const int t = __ffs(int(B)) - 1;
+    if (t > 2) return;
+    const std::uint32_t odd = B >> t;
+    std::uint32_t inv = odd;  // 1 / B' mod 2^32 by Newton's iteration (3 bits to begin with)
+    for (int i = 0; i < 4; ++i) inv *= 2u - odd * inv;
+    const float b = __uint_as_float((std::uint32_t(127 + eb) << 23) | (B & 0x7fffffu));
+    const RecipF rb(b);
+    for (int r = -7; r <= 7; r += 2) {
+        if ((r < 0 ? -r : r) << t > 7) continue;
+        for (int k = 24; k <= 25; ++k)
+            for (std::uint32_t j = 0; j < (1u << t); ++j) {
+                const std::uint32_t low = (std::uint32_t(-r) * inv) & ((1u << (k - t)) - 1u);
+                std::uint32_t M = low + (j << (k - t));
+                if (k == 24) M |= 1u << 24;
+                if (M < (1u << 24)) continue;
+                const unsigned long long num = (unsigned long long)B * M + (unsigned long long)((long long)r * (1 << t));
+                const std::uint32_t A = std::uint32_t(num >> k);
+                if (A < 0x800000u || A > 0xffffffu) continue;
+                const float a = __uint_as_float((std::uint32_t(127 + ea) << 23) | (A & 0x7fffffu));
+                count(HARD, bits_equal(rb(a), a / b));
+                count(HARD, bits_equal(rb(-a), -a / b));
+            }
+    }
 }
 
 __global__ void sixths(int e) {
@@ -41,6 +74,37 @@ __global__ void newton(int e) {
     atomicMax(&g_milli[1], (unsigned long long)ceil(1000.0 * fabs(fma(-s, s, x) / (2.0 * s)) / ulp(s)));
 }
 
+// Steps of states whose momenta, or whose constant L, go down to the subnormals.
+__global__ void tiny() {
+    std::uint32_t s = mix(blockIdx.x * blockDim.x + threadIdx.x + 4242u);
+    auto uni = [&]() {
+        s = mix(s + 0x9e3779b9u);
+        return float(s >> 8) * 0x1p-24f;
+    };
+    auto small = [&](float top) {
+        const float u = uni(), x = u < 0.3f ? top * uni() : top * exp2f(-126.0f * uni());
+        return u > 0.97f ? 0.0f : (uni() < 0.5f ? -x : x);
+    };
+    View<float> v;
+    v.M = 1.0f;
+    v.a = uni() < 0.5f ? 0.0f : uni();
+    v.a2 = v.a * v.a;
+    v.twoM = v.rs = 2.0f;
+    v.shared_div = 1u;
+    const float r = 2.1f + 58.0f * uni(), th = 0.05f + 3.04f * uni(), h = 0.05f + 0.45f * uni(), E = 0.8f + 0.4f * uni();
+    auto near = [](float a, float b) { return a == b || fabsf(a - b) <= 0x1p-100f; };
+    KS<float> y{r, th, 0.1f + 6.0f * uni(), small(1.0f), small(1.0f)}, z = y;
+    const KC<float> c = make_kc<float>(v, E, small(4.0f));
+    kerr_step_ref(y, h, v, c);
+    kerr_rk4_ref_div(z, h, v, c);
+    count(TINY_KERR, y.r == z.r && y.th == z.th && y.ph == z.ph && near(y.pr, z.pr) && near(y.pth, z.pth));
+    SS<float> p{r, th, 0.1f + 6.0f * uni(), 1.0f + uni(), small(0.5f), small(0.05f), small(0.05f)}, q = p;
+    schw_step(p, h, v);
+    schw_rk4_div(q, h, v.rs);
+    count(TINY_SCHW, p.r == q.r && p.th == q.th && p.ph == q.ph && p.ut == q.ut && near(p.ur, q.ur) &&
+                         near(p.uth, q.uth) && near(p.uph, q.uph));
+}
+
 #define CHECK(call)                                                                              \
     do {                                                                                         \
         const cudaError_t e_ = (call);                                                           \
@@ -53,6 +117,11 @@ __global__ void newton(int e) {
 int main() {
     if (division_main() != 0) return 1;
     CHECK(cudaGetLastError());  // any launch or copy of it that was refused
+    for (int ea : {-102, -30, 0, 60})
+        for (int eb : {-60, -1, 0, 20}) {
+            hard<<<(1 << 23) / 256, 256>>>(ea, eb);
+            CHECK(cudaGetLastError());
+        }
     for (int e : {-102, -80, 0, 100, 127}) {
         sixths<<<(1 << 23) / 256, 256>>>(e);
         CHECK(cudaGetLastError());
@@ -61,6 +130,8 @@ int main() {
         newton<<<(1 << 23) / 256, 256>>>(e);
         CHECK(cudaGetLastError());
     }
+    tiny<<<(1 << 22) / 256, 256>>>();
+    CHECK(cudaGetLastError());
     CHECK(cudaDeviceSynchronize());
     unsigned long long miss[N_CHECKS], done[N_CHECKS], milli[2];
     CHECK(cudaMemcpyFromSymbol(miss, g_miss, sizeof(miss)));

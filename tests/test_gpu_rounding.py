@@ -1,9 +1,17 @@
-"""The kernels' divisions by 6, reciprocals and roots.
+"""The kernels' quotients, reciprocals and roots where they are hardest.
 
 tests/rounding_check.cu runs tests/division_check.cu with every launch and copy
 checked and counts what it compares itself.
 
-* x / 6 is the compiled quotient bit for bit from 2^-102 (FP32) and 2^-968 (FP64).
+* Quotients of the shared reciprocals are the compiled ones bit for bit for
+  numerators of 2^-102 and more, for every divisor also the quotients within
+  seven of the smallest distances from the midpoint of two floats; x / 6 likewise from 2^-102 (FP32) and 2^-968
+  (FP64).
+* Smaller numerators lose part of their remainder, so a quotient may be off by
+  one unit in its last place: with radii from 2.1 M and sin(theta) above 0.05 the
+  divisors are 2^-13 and more, which is 2^-112 for each of six quotients.  Steps
+  with momenta down to the subnormals therefore give the same positions, and
+  momenta within 2^-100.
 * The SFU's 20-bit reciprocal and reciprocal root are within 2^-19 (2^-20 by the
   bits of the operand that they read, 2^-20 by those that they return); one
   cubic step leaves 2^-57, 0.0625 units in the last place, beside the last
@@ -15,10 +23,11 @@ from __future__ import annotations
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
-SIXTH_F, SIXTH_D = range(2)
+HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW = range(5)
 
 
 def _build(tmp_path):
@@ -27,6 +36,28 @@ def _build(tmp_path):
     subprocess.run([B._nvcc(), *B.ARCH, *B.NVCC_FLAGS, str(ROOT / "tests" / "rounding_check.cu"), "-o", str(exe)],
                    check=True, capture_output=True, text=True)
     return exe
+
+
+def _hard_numerators():
+    """How many numerators one launch of the program's hard() has."""
+    u64, n = np.uint64, 0
+    for t in range(3):
+        odd = np.arange((0x800000 >> t) | 1, 0x1000000 >> t, 2, dtype=u64)
+        B, inv = odd << u64(t), odd.copy()
+        for _ in range(4):
+            inv = (inv * ((u64(2) - odd * inv) & u64(0xffffffff))) & u64(0xffffffff)
+        for r in (r for r in range(-7, 8, 2) if abs(r) << t <= 7):
+            for k in (24, 25):
+                low = (u64(-r % (1 << 32)) * inv) & u64((1 << (k - t)) - 1)
+                for j in range(1 << t):
+                    M = low + u64(j << (k - t))
+                    if k == 24:
+                        M |= u64(1 << 24)
+                    num = B * M + u64((r << t) % (1 << 64))
+                    assert not np.any(num & u64((1 << k) - 1))
+                    A = num >> u64(k)
+                    n += int(np.sum((M >= 1 << 24) & (A >= 0x800000) & (A <= 0xffffff)))
+    return n
 
 
 def test_no_gpu_is_no_pass(tmp_path):
@@ -44,7 +75,9 @@ def test_rounding(tmp_path, sgx):
     old, new = ([int(x) for x in line.split()] for line in run.stdout.strip().splitlines())
     print(old, new)
     assert old[:7] == [0] * 7 and max(old[7:9]) <= 1 and old[9] <= 8
-    miss, done, milli = new[0:4:2], new[1:4:2], new[4:]
+    miss, done, milli = new[0:10:2], new[1:10:2], new[10:]
+    assert done[HARD] == 2 * 16 * _hard_numerators()
     assert done[SIXTH_F] == done[SIXTH_D] == 5 << 23
-    assert miss == [0] * 2
+    assert done[TINY_KERR] == done[TINY_SCHW] == 1 << 22
+    assert miss == [0] * 5
     assert 450 < min(milli) and max(milli) <= 570
