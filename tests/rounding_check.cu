@@ -2,13 +2,14 @@
 // with its launches and copies checked, and the same arithmetic where it is
 // hardest or leaves the ordinary: quotients nearest to a rounding boundary,
 // the ends of the exponent range, x / 6 in FP64, momenta and angular momenta down
-// to the subnormals.  Every kernel counts what it compared.  Prints division_check's line, then mismatches,
+// to the subnormals, roots of subnormals, differences that are not finite.  Every
+// kernel counts what it compared.  Prints division_check's line, then mismatches,
 // comparisons and worst errors (in thousandths of a unit in the last place).
 #define main division_main
 #include "division_check.cu"
 #undef main
 
-enum { HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW, N_CHECKS };
+enum { HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW, ROOT, NORM, N_CHECKS };
 __device__ unsigned long long g_miss[N_CHECKS], g_done[N_CHECKS], g_milli[2];
 
 __device__ __forceinline__ void count(int k, bool ok) {
@@ -17,7 +18,7 @@ __device__ __forceinline__ void count(int k, bool ok) {
 }
 __device__ __forceinline__ bool bits_equal(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
 __device__ __forceinline__ bool bits_equal(double a, double b) {
-    return __double_as_longlong(a) == __double_as_longlong(b);
+    return __double_as_longlong(a) == __double_as_longlong(b) || (isnan(a) && isnan(b));
 }
 
 // For every divisor significand B the numerators A with A 2^k = B M + r, M odd of
@@ -105,6 +106,51 @@ __global__ void tiny() {
                          near(p.uth, q.uth) && near(p.uph, q.uph));
 }
 
+// p_theta on the Carter constant (Theta = Q with cos theta = 0) for Theta of every kind.
+__global__ void roots() {
+    const int i = threadIdx.x;
+    const double kinds[] = {0.0, -0.0, -1.0, 5e-324, 1e-310, 2.2250738585072009e-308, 2.2250738585072014e-308, 1e-300, 0.25,
+                            4.0, 1e300, 1.7976931348623157e308, __longlong_as_double(0x7ff0000000000000ll),
+                            __longlong_as_double((long long)0xfff0000000000000ull)};
+    if (i >= int(sizeof(kinds) / sizeof(kinds[0]))) return;
+    KC<double> k{};
+    const double th = kinds[i], got = project_pth(-3.0, 1.0, 0.0, th, k), want = copysign(th > 0.0 ? sqrt(th) : 0.0, -3.0);
+    const long long d = __double_as_longlong(got) - __double_as_longlong(want);
+    count(ROOT, d >= -1 && d <= 1);
+}
+
+// The FP64 norm with one difference, or its scale, not finite or too large: 1e30 where a
+// difference is NaN or infinite or its quotient beyond 1e30, the other components'
+// norm where only a scale is infinite.
+__global__ void odd_norms() {
+    std::uint32_t s = mix(blockIdx.x * blockDim.x + threadIdx.x + 31337u);
+    auto uni = [&]() {
+        s = mix(s + 0x9e3779b9u);
+        return double(s >> 8) * 0x1p-24;
+    };
+    const int which = int(uni() * 6.0), kind = int(uni() * 8.0);
+    const long long specials[] = {0x7ff8000000000000ll, (long long)0xfff8000000000000ull, 0x7ff0000000000001ll,
+                                  0x7fffffffffffffffll, 0x7ff0000000000000ll, (long long)0xfff0000000000000ull};
+    double y[6], y4[6], k4[6], k5[6];
+    for (int i = 0; i < 6; ++i) {
+        y[i] = 4.0 * uni() - 2.0;
+        y4[i] = y[i] * (1.0 + 0.01 * uni());
+        k4[i] = 2.0 * uni() - 1.0;
+        k5[i] = k4[i] - exp2(-40.0 * uni());
+    }
+    if (kind < 6) (uni() < 0.5 ? k4 : k5)[which] = __longlong_as_double(specials[kind]);
+    else if (kind == 6) k4[which] = 1e200;
+    else y4[which] = __longlong_as_double(0x7ff0000000000000ll);
+    auto six = [](const double* v) { return KSC<double>{v[0], v[1], v[2], v[3], v[4], v[5]}; };
+    const KAttempt<double> A{six(y4), six(k4), six(k5), 0.015625};
+    double want = 0.0;
+    for (int i = 0; i < 6; ++i)
+        want = fmax(want, fabs(A.h6 * (k4[i] - k5[i])) / (double(1e-6f) * (1.0 + fmax(fabs(y[i]), fabs(y4[i])))));
+    if (kind < 7) want = 1e30;
+    const long long d = __double_as_longlong(error_norm_pos(six(y), A, 1e-6f)) - __double_as_longlong(want);
+    count(NORM, kind < 7 ? d == 0 : d >= -8 && d <= 8);
+}
+
 #define CHECK(call)                                                                              \
     do {                                                                                         \
         const cudaError_t e_ = (call);                                                           \
@@ -131,6 +177,10 @@ int main() {
         CHECK(cudaGetLastError());
     }
     tiny<<<(1 << 22) / 256, 256>>>();
+    CHECK(cudaGetLastError());
+    roots<<<1, 32>>>();
+    CHECK(cudaGetLastError());
+    odd_norms<<<(1 << 20) / 256, 256>>>();
     CHECK(cudaGetLastError());
     CHECK(cudaDeviceSynchronize());
     unsigned long long miss[N_CHECKS], done[N_CHECKS], milli[2];

@@ -16,6 +16,10 @@ checked and counts what it compares itself.
   bits of the operand that they read, 2^-20 by those that they return); one
   cubic step leaves 2^-57, 0.0625 units in the last place, beside the last
   rounding's 0.5, two quadratic ones of the root less: 0.57 in all.
+* A root is the library's within one unit in the last place, of subnormals,
+  infinity and negative numbers too.
+* A difference that is not finite makes the FP64 error norm 1e30, whatever sign a
+  NaN has.
 """
 
 from __future__ import annotations
@@ -27,7 +31,7 @@ import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
-HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW = range(5)
+HARD, SIXTH_F, SIXTH_D, TINY_KERR, TINY_SCHW, ROOTS, NORM = range(7)
 
 
 def _build(tmp_path):
@@ -75,9 +79,10 @@ def test_rounding(tmp_path, sgx):
     old, new = ([int(x) for x in line.split()] for line in run.stdout.strip().splitlines())
     print(old, new)
     assert old[:7] == [0] * 7 and max(old[7:9]) <= 1 and old[9] <= 8
-    miss, done, milli = new[0:10:2], new[1:10:2], new[10:]
+    miss, done, milli = new[0:14:2], new[1:14:2], new[14:]
     assert done[HARD] == 2 * 16 * _hard_numerators()
     assert done[SIXTH_F] == done[SIXTH_D] == 5 << 23
     assert done[TINY_KERR] == done[TINY_SCHW] == 1 << 22
-    assert miss == [0] * 5
+    assert done[ROOTS] == 14 and done[NORM] == 1 << 20
+    assert miss == [0] * 7
     assert 450 < min(milli) and max(milli) <= 570
