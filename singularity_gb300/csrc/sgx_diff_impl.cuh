@@ -51,7 +51,7 @@ constexpr std::uint64_t kSmallForward = 1u << 18, kSmallBackward = 1u << 16;  //
 // Warps an SM has to hold in the backward kernels (their comment says why).
 template <class T, bool SLAB, bool DUALJ, int CK>
 constexpr int kBackwardWarps = sizeof(T) == 8 || DUALJ ? 8 : CK == kCkDense ? 10 : SLAB ? 12 : 16;
-constexpr std::uint64_t kOneWaveBackward = 8 * 32 * 152;  // rays that 8 warps an SM hold at once
+constexpr std::uint64_t kOneWaveRaysPerSm = 8 * 32;  // rays that 8 warps hold at once
 constexpr int kMaxCross = 8;  // crossings recorded per ray (crossing model)
 constexpr int NS = 8;         // state: r, theta, phi, p_r, p_theta, psi (swept angle), sin(theta), cos(theta)
 constexpr int NC = NS + 1;    // checkpoint: state and transmittance
@@ -846,8 +846,8 @@ __device__ __forceinline__ void step_adjoint(const T* yp, T E, T L, T a, const D
 // registers for more of them in flight are worth more than warps.  Backward call
 // on one GB300, ms, at W = 16 (128 registers) / W = 10 (168, 12 warps resident):
 // one-warp blocks 160 x 96 x 4 spp 0.80 / 0.59, 255 x 193 crossings 0.57 / 0.50;
-// 128-thread blocks 512 x 512 x 4 6.38 / 6.05.  Up to 38,912 rays 8 warps an SM
-// hold them all at once, and 224 registers take 64 x 64 x 4 from 0.34 to 0.32;
+// 128-thread blocks 512 x 512 x 4 6.38 / 6.05.  Up to 256 rays an SM (38,912
+// on its 152) 8 warps hold them all at once, and 224 registers take 64 x 64 x 4 from 0.34 to 0.32;
 // above that line they need a second wave (160 x 96 x 4: 0.71).  In the sparse
 // form W = 12 takes the slab from 6.61 to 6.48, but the crossings, whose segment
 // is their main traffic, from 1.63 to 1.65: they stay at 16.  The dual numbers
@@ -1311,13 +1311,17 @@ cudaError_t run_backward(sgx_diff_state& st, const float* gimg, double* d_out4, 
         if (dense) {
             const int smem = (kCkDense + 1) * NC * th * int(sizeof(T));
             constexpr int kW = kBackwardWarps<T, false, false, kCkDense>;
+            int dev = 0, sms = 0;
+            cudaError_t e = cudaGetDevice(&dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return e;
             auto* kern = !slab && !st.xs ? diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, kW, false>
-                         : st.n > kOneWaveBackward
+                         : st.n > kOneWaveRaysPerSm * std::uint64_t(sms)
                              ? (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads>
                                      : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads>)
                              : (slab ? diff_backward_kernel<T, true, false, kCkDense, kSmallThreads, 8>
                                      : diff_backward_kernel<T, false, false, kCkDense, kSmallThreads, 8>);
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             kern<<<grid, th, smem, s>>>(k, p, b, gimg);
         }
